@@ -748,7 +748,8 @@ int gbn_run(gbn_handle h, void* stream, gbn_state* st, int32_t num_iterations, i
     } else {
       HierView hv{h->m.y, h->m.hier_sinv, h->m.hier_cmodel, h->m.offsets, h->m.chains_per_model, h->m.num_models,
                   (float)(1.0 / (h->m.hyper[0] * h->m.hyper[0])), (float)(1.0 / h->m.hyper[1])};
-      launch_persistent_hier(h->dP, hv, h->counters + 7, h->order, h->C, h->hp.dense != 0, s);
+      launch_persistent_hier(h->dP, hv, h->counters + 7, h->order, h->C, h->D, h->maxd, h->cfg.algo == GBN_ALGO_NUTS,
+                             h->hp.dense != 0, s);
     }
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -845,7 +846,8 @@ int gbn_sample_async(gbn_handle h, void* stream, gbn_state* st) {
     } else {
       HierView hv{h->m.y, h->m.hier_sinv, h->m.hier_cmodel, h->m.offsets, h->m.chains_per_model, h->m.num_models,
                   (float)(1.0 / (h->m.hyper[0] * h->m.hyper[0])), (float)(1.0 / h->m.hyper[1])};
-      launch_persistent_hier(h->dP, hv, h->counters + 7, h->order, h->C, h->hp.dense != 0, s);
+      launch_persistent_hier(h->dP, hv, h->counters + 7, h->order, h->C, h->D, h->maxd, h->cfg.algo == GBN_ALGO_NUTS,
+                             h->hp.dense != 0, s);
     }
   } else {
     e = cudaMemsetAsync(h->async_iter, 0, sizeof(int32_t), s);

@@ -26,6 +26,8 @@
 //   _nuts_next :416-455, sample_kernel :459-530.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "hier_potential.cuh"
 #include "internal.h"
@@ -966,6 +968,12 @@ __device__ __forceinline__ const AdvParams& stage_params(const AdvParams* __rest
   return *sp;
 }
 
+}  // namespace gbn
+
+#include "hier_engine.cuh"
+
+namespace gbn {
+
 template <int NT, bool DM>
 __global__ void __launch_bounds__(256) advance_kernel(const AdvParams* __restrict__ Pp, int parity) {
   __shared__ double red[16];
@@ -1231,11 +1239,54 @@ __global__ void __launch_bounds__(256) persistent_sv_kernel(const AdvParams* __r
 }
 
 // --------------------------------------------------------------------- launchers
+// Shared memory of an SM for its chains' U-turn checkpoints (64, 96 and 180 KB: no faster).
+constexpr size_t HIER_CK_SMEM = 128 * 1024;
+
+template <int K>
+static void launch_hier_reg(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order, int C,
+                            int maxd, int sms, int optin, cudaStream_t st) {
+  // few chains: a warp per SM before any SM takes two
+  const int warps = C <= sms ? 1 : (C <= 2 * sms ? 2 : 4);
+  const int resident = 12 / warps;  // CTAs per SM that the checkpoints' shared memory leaves room for
+  const size_t slot = sizeof(float) * 64 * K * warps;
+  const int need = (C + warps - 1) / warps;
+  const int per_sm_needed = std::min(resident, (need + sms - 1) / sms);
+  const size_t budget = std::min((size_t)(HIER_CK_SMEM / per_sm_needed), (size_t)optin - 2048);
+  const int slots = (int)std::min((size_t)maxd, budget / slot);
+  const size_t smem = slot * slots;
+  cudaFuncSetAttribute(persistent_hier_reg_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int blocks = need;
+  if (need > sms) {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_reg_kernel<K>, 32 * warps, smem);
+    blocks = std::min(need, sms * std::max(per_sm, 1));
+  }
+  persistent_hier_reg_kernel<K><<<blocks, 32 * warps, smem, st>>>(dP, hv, queue_head, order, slots * 64 * K);
+}
+
 void launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order,
-                            int C, bool dense, cudaStream_t st) {
-  int dev = 0, sms = 0, per_sm = 0;
+                            int C, int D, int maxd, bool nuts, bool dense, cudaStream_t st) {
+  int dev = 0, sms = 0, per_sm = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  // The register engine holds up to 288 dimensions (nine elements a lane); HMC, dense mass matrices and
+  // larger models run the state machine over memory.
+  if (nuts && !dense && D <= 288) {
+    if (D <= 32)
+      launch_hier_reg<1>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
+    else if (D <= 64)
+      launch_hier_reg<2>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
+    else if (D <= 96)
+      launch_hier_reg<3>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
+    else if (D <= 160)
+      launch_hier_reg<5>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
+    else if (D <= 224)
+      launch_hier_reg<7>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
+    else
+      launch_hier_reg<9>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
+    return;
+  }
   if (dense)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_kernel<true>, 256, 0);
   else
