@@ -1,0 +1,380 @@
+// logreg_fp32.cuh -- FP32 CUDA-core kernel of the logistic-regression potential.
+//
+//   l = X b;  U = sum_n [softplus(l_n) - y_n l_n] + prior;  dU/db = X^T (sigmoid(l) - y) + prior
+// Fused per row tile: logits -> (softplus, sigmoid) -> gradient, so no logit reaches memory.  A CTA
+// owns CT chains and a strided set of RT-row tiles; a thread holds 4 RG rows x 4 CG chains of logits.
+//
+// Bound: FP32 instruction issue.  A logit costs 2 p fused multiply-adds and ~60 instructions of expf, log1pf
+// and reciprocal (~100 with the compiler's division: 1 + e^-|l| lies in [1, 2], so the reciprocal needs no
+// range handling, recip_1_2).  The multiply-adds run as FP32x2 over pairs of chains: no more per cycle than
+// scalar ones, but half the issue slots, which the epilogues of the other warps use.  Operands come from
+// shared memory as 16-byte words; X tiles arrive by cp.async one tile ahead, rows swizzled by groups of
+// four so that the eight lanes of a load phase meet eight bank groups.
+// Measured at 581,012 x 55 x 1,024 chains: 5.52 ms (64 x 64 tile, 4 x 4 a thread, X through registers and a
+// transposed copy) -> 3.64 ms = 36 TFLOP/s.  8 x 8 logits a thread with 8 warps per SM: 3.85; scalar
+// multiply-adds: 3.86.
+// Sums: a chain's log-likelihood of four consecutive rows in FP32, then compensated FP32 over the
+// thread's rows and float-float across threads; FP64 across CTAs.
+#pragma once
+#include <algorithm>
+
+#include "common.cuh"
+#include "internal.h"
+
+namespace gbn {
+
+// 1 / d for d in [1, 2], rounded to nearest: one Newton-Raphson step on the approximate reciprocal with
+// the residual exact in a fused multiply-add (Markstein, IBM J. Res. Dev. 34, 1990).  Equal to 1.0f / d
+// for each of the 2^23 + 1 floats of the range (compared on the GPU).
+__device__ __forceinline__ float recip_1_2(float d) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return fmaf(y, fmaf(-d, y, 1.0f), y);
+}
+
+struct LogregArgs {
+  const float* x;  // [n][p]
+  const float* y;
+  int64_t n;
+  int p;
+  const float* q;  // [npts][ld]
+  int npts, ld;
+  float* part_g;    // [gridDim.y][npts][64]
+  double* part_ll;  // [gridDim.y][npts]
+  const int32_t* pending;
+};
+
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(in ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(in ? 16 : 0)
+               : "memory");
+}
+
+// CT chains, NTH threads, RG groups of 4 rows and CG groups of 4 chains a thread in the logit phase,
+// 4 CG chains x 4 FG features a thread in the gradient phase, SP floats a row of the X tile (32 or 64),
+// NB tile buffers.
+template <int CT, int NTH, int RG, int CG, int FG, int SP, int NB>
+struct LogregTile {
+  static constexpr int TX = CT / (4 * CG), TY = NTH / TX, RT = 4 * RG * TY;
+  static constexpr size_t bytes(int dp) {
+    return sizeof(float) * (size_t)(NB * RT * SP + dp * CT + RT * CT + NB * RT) + sizeof(float2) * (NTH / 32) * CT;
+  }
+};
+
+template <int CT, int NTH, int RG, int CG, int FG, int SP, int NB, int MINB>
+__global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs A) {
+  if (A.pending && *A.pending == 0) return;
+  using T = LogregTile<CT, NTH, RG, CG, FG, SP, NB>;
+  constexpr int TX = T::TX, TY = T::TY, RT = T::RT;
+  extern __shared__ __align__(16) float lr_smem[];
+  const int p = A.p, nc = (p + 3) >> 2;
+  float* const xs = lr_smem;                 // [NB][RT][SP], chunk c of row r at c ^ ((r >> 2) & 7)
+  float* const es = xs + NB * RT * SP;       // [RT][CT]
+  float* const ys = es + RT * CT;            // [NB][RT]
+  float2* const lls = reinterpret_cast<float2*>(ys + NB * RT);  // [NTH / 32][CT]
+  float* const bs = reinterpret_cast<float*>(lls + (NTH / 32) * CT);  // [4 nc][CT]
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  const int c0 = blockIdx.x * CT, rg = blockIdx.y, groups = gridDim.y;
+  const int64_t ntiles = (A.n + RT - 1) / RT;
+
+  for (int k = tid; k < NB * RT * SP; k += NTH) xs[k] = 0.0f;  // features past p stay zero
+  for (int k = tid; k < 4 * nc * CT; k += NTH) {
+    const int c = k / (4 * nc), d = k % (4 * nc);
+    bs[d * CT + c] = (d < p && c0 + c < A.npts) ? A.q[(size_t)(c0 + c) * A.ld + d] : 0.0f;
+  }
+  __syncthreads();
+  auto load_tile = [&](int64_t tile, int buf) {
+    float* const dst = xs + buf * RT * SP;
+    const int64_t r0 = tile * RT;
+    const float* const src = A.x + r0 * p;
+    const int64_t left = A.n - r0;
+    if ((p & 3) == 0 && (reinterpret_cast<uintptr_t>(A.x) & 15) == 0) {
+      const int q4 = p >> 2;
+      for (int k = tid; k < RT * q4; k += NTH) {
+        const int r = k / q4, c = k - r * q4;
+        const bool in = r < left;
+        cp_async16(dst + r * SP + ((c ^ ((r >> 2) & 7)) << 2), in ? src + (size_t)r * p + 4 * c : A.x, in);
+      }
+    } else {
+      int r = tid / p, d = tid - r * p;
+      const int sr = NTH / p, sd = NTH - sr * p;
+      for (int k = tid; k < RT * p; k += NTH) {
+        const bool in = r < left;
+        cp_async4(dst + r * SP + (((d >> 2) ^ ((r >> 2) & 7)) << 2) + (d & 3), in ? src + k : A.x, in);
+        r += sr;
+        d += sd;
+        if (d >= p) {
+          d -= p;
+          ++r;
+        }
+      }
+    }
+    for (int r = tid; r < RT; r += NTH) cp_async4(ys + buf * RT + r, r < left ? A.y + r0 + r : A.y, r < left);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  // Gradient phase: a thread owns 4 CG chains x 4 FG features and takes the rows in order, so the sum of
+  // an output does not depend on the tile's shape (only on which 64-row tiles a row group holds).
+  const int dgn = (nc + FG - 1) / FG, outs = TX * dgn;
+  const int gc = tid % TX, gd = tid / TX;
+  static_assert(TX * (SP / (4 * FG)) <= NTH, "an output tile per thread");
+  float2 gacc[2 * CG][4 * FG];  // pairs of chains
+#pragma unroll
+  for (int i = 0; i < 2 * CG; ++i)
+#pragma unroll
+    for (int j = 0; j < 4 * FG; ++j) gacc[i][j] = make_float2(0.0f, 0.0f);
+  Comp32 ll[4 * CG];
+#pragma unroll
+  for (int j = 0; j < 4 * CG; ++j) ll[j] = Comp32{0.0f, 0.0f};
+
+  int buf = 0;
+  if (rg < ntiles) load_tile(rg, 0);
+  for (int64_t tile = rg; tile < ntiles; tile += groups, buf ^= NB - 1) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // this tile has landed; every thread is done with the other buffer and with E
+    if (NB == 2 && tile + groups < ntiles) load_tile(tile + groups, buf ^ 1);
+    const float* const xb = xs + buf * RT * SP;
+    // ------------------------------------------------ logits
+    float2 acc[4 * RG][2 * CG];  // pairs of chains
+#pragma unroll
+    for (int i = 0; i < 4 * RG; ++i)
+#pragma unroll
+      for (int j = 0; j < 2 * CG; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+    for (int c = 0; c < nc; ++c) {
+      float4 xv[4 * RG];
+#pragma unroll
+      for (int g = 0; g < RG; ++g)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          xv[4 * g + i] = *reinterpret_cast<const float4*>(xb + (4 * (g * TY + ty) + i) * SP +
+                                                           ((c ^ ((g * TY + ty) & 7)) << 2));
+#pragma unroll
+      for (int dd = 0; dd < 4; ++dd) {
+        float2 b[2 * CG];
+#pragma unroll
+        for (int h = 0; h < CG; ++h) {
+          const float4 b4 = *reinterpret_cast<const float4*>(bs + (4 * c + dd) * CT + h * (CT / CG) + 4 * tx);
+          b[2 * h] = make_float2(b4.x, b4.y);
+          b[2 * h + 1] = make_float2(b4.z, b4.w);
+        }
+#pragma unroll
+        for (int i = 0; i < 4 * RG; ++i) {
+          const float xa = dd == 0 ? xv[i].x : (dd == 1 ? xv[i].y : (dd == 2 ? xv[i].z : xv[i].w));
+#pragma unroll
+          for (int j = 0; j < 2 * CG; ++j) acc[i][j] = __ffma2_rn(make_float2(xa, xa), b[j], acc[i][j]);
+        }
+      }
+    }
+    // ------------------------------------------------ softplus and sigmoid
+    const int64_t left = A.n - tile * RT;
+#pragma unroll
+    for (int g = 0; g < RG; ++g) {
+      float llt[4 * CG];
+#pragma unroll
+      for (int j = 0; j < 4 * CG; ++j) llt[j] = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = 4 * (g * TY + ty) + i;
+        const float yy = ys[buf * RT + r];
+        const bool in = r < left;
+        float ev[4 * CG];
+#pragma unroll
+        for (int j = 0; j < 4 * CG; ++j) {
+          const float l = (j & 1) ? acc[4 * g + i][j >> 1].y : acc[4 * g + i][j >> 1].x;
+          const float t = expf(-fabsf(l));
+          const float sp = fmaxf(l, 0.0f) + log1pf(t);
+          const float inv = recip_1_2(1.0f + t);
+          const float sig = (l >= 0.0f) ? inv : t * inv;
+          ev[j] = in ? sig - yy : 0.0f;
+          llt[j] += in ? sp - yy * l : 0.0f;
+        }
+#pragma unroll
+        for (int h = 0; h < CG; ++h)
+          *reinterpret_cast<float4*>(es + r * CT + h * (CT / CG) + 4 * tx) =
+              make_float4(ev[4 * h], ev[4 * h + 1], ev[4 * h + 2], ev[4 * h + 3]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4 * CG; ++j) ll[j].add(llt[j]);
+    }
+    __syncthreads();
+    // ------------------------------------------------ gradient
+    if (tid < outs) {
+#pragma unroll 2
+      for (int r = 0; r < RT; ++r) {
+        float2 e[2 * CG];
+        float xf[4 * FG];
+#pragma unroll
+        for (int h = 0; h < CG; ++h) {
+          const float4 e4 = *reinterpret_cast<const float4*>(es + r * CT + h * (CT / CG) + 4 * gc);
+          e[2 * h] = make_float2(e4.x, e4.y);
+          e[2 * h + 1] = make_float2(e4.z, e4.w);
+        }
+#pragma unroll
+        for (int f = 0; f < FG; ++f) {
+          const float4 x4 =
+              *reinterpret_cast<const float4*>(xb + r * SP + (((gd * FG + f) ^ ((r >> 2) & 7)) << 2));
+          xf[4 * f] = x4.x; xf[4 * f + 1] = x4.y; xf[4 * f + 2] = x4.z; xf[4 * f + 3] = x4.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 4 * FG; ++j)
+#pragma unroll
+          for (int i = 0; i < 2 * CG; ++i) gacc[i][j] = __ffma2_rn(e[i], make_float2(xf[j], xf[j]), gacc[i][j]);
+      }
+    }
+    if (NB == 1 && tile + groups < ntiles) {
+      __syncthreads();
+      load_tile(tile + groups, 0);
+    }
+  }
+  // ------------------------------------------------ the CTA's partials
+  if (tid < outs) {
+#pragma unroll
+    for (int i = 0; i < 4 * CG; ++i) {
+      const int c = c0 + (i >> 2) * (CT / CG) + 4 * gc + (i & 3);
+      if (c >= A.npts) continue;
+#pragma unroll
+      for (int f = 0; f < FG; ++f) {
+        const float2* const v = gacc[i >> 1] + 4 * f;
+        *reinterpret_cast<float4*>(A.part_g + ((size_t)rg * A.npts + c) * 64 + 4 * (gd * FG + f)) =
+            (i & 1) ? make_float4(v[0].y, v[1].y, v[2].y, v[3].y) : make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4 * CG; ++j) {
+    FF v = comp_ff(ll[j]);
+#pragma unroll
+    for (int o = 16; o >= TX; o >>= 1) v = ff_add(v, ff_shfl_xor(v, o));
+    if ((tid & 31) < TX) lls[(tid >> 5) * CT + (j >> 2) * (CT / CG) + 4 * tx + (j & 3)] = make_float2(v.hi, v.lo);
+  }
+  __syncthreads();
+  if (tid < CT && c0 + tid < A.npts) {
+    FF v{lls[tid].x, lls[tid].y};
+    for (int w = 1; w < NTH / 32; ++w) v = ff_add(v, FF{lls[w * CT + tid].x, lls[w * CT + tid].y});
+    A.part_ll[(size_t)rg * A.npts + c0 + tid] = ff_value(v);
+  }
+}
+
+// Row tiles of 64 rows: up to this many, every tile is a row group of its own and the finish adds them in
+// order, so a small data set's gradient is one fixed sum whatever the launch shape.
+constexpr int LR_ORDERED = 128;
+
+// The sums over row groups and the prior for one chain, a CTA of 256 threads.  By one warp the loads of
+// ~150 row groups (a few-chain launch) took 29 us in dependent rounds of eight.
+__global__ void __launch_bounds__(256) logreg_fp32_finish_kernel(const LogregArgs A, int groups, float inv_var,
+                                                                 double pe_const, double* __restrict__ pe,
+                                                                 float* __restrict__ g) {
+  if (A.pending && *A.pending == 0) return;
+  __shared__ float4 part[LR_ORDERED][16];
+  const int c = blockIdx.x, tid = threadIdx.x, d4 = tid & 15, slice = tid >> 4;
+  const float4* const src = reinterpret_cast<const float4*>(A.part_g + (size_t)c * 64) + d4;
+  const bool ordered = groups <= LR_ORDERED;
+  if (4 * d4 < A.p) {
+    if (ordered) {
+#pragma unroll 8
+      for (int r = slice; r < groups; r += 16) part[r][d4] = src[(size_t)r * A.npts * 16];
+    } else {  // 16 slices of the row groups, each in order
+      float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
+      for (int r = slice; r < groups; r += 16) {
+        const float4 v = src[(size_t)r * A.npts * 16];
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
+      part[slice][d4] = s;
+    }
+  }
+  if (tid < 32) {  // potential and prior, in FP64 as logreg_finish_warp
+    double lp = 0.0, lsum = 0.0;
+    for (int d = tid; d < A.p; d += 32) {
+      const double b = (double)A.q[(size_t)c * A.ld + d];
+      lp += 0.5 * b * b * (double)inv_var;
+    }
+    for (int r = tid; r < groups; r += 32) lsum += A.part_ll[(size_t)r * A.npts + c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lp += __shfl_xor_sync(0xffffffffu, lp, o);
+      lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    }
+    if (tid == 0) pe[c] = lsum + lp + pe_const;
+  }
+  __syncthreads();
+  if (tid >= 64 && tid < 128) {  // not the warp that sums in FP64
+    const int d = tid - 64, rows = ordered ? groups : 16;
+    if (d < A.p) {
+      const float* const col = reinterpret_cast<const float*>(&part[0][0]) + d;
+      float t = 0.0f;
+#pragma unroll 16
+      for (int k = 0; k < rows; ++k) t += col[k * 64];
+      g[(size_t)c * A.ld + d] = fmaf(A.q[(size_t)c * A.ld + d], inv_var, t);
+    }
+  }
+}
+
+// ------------------------------------------------------------------ launch shapes
+// The widest tile whose CTAs still fill the chip: 128 chains (4 x 8 logits a thread, 256 threads), 64 (4 x 4,
+// 256 threads), 16 and, for the few chains of an ordinary run, 8 (a warp); 64 rows each.
+struct LogregShape {
+  int variant, ct, per_sm;
+};
+inline LogregShape logreg_fp32_shape(int64_t n, int npts) {
+  const int64_t tiles = (n + 63) / 64;
+  if (npts > 64 && (npts + 127) / 128 * tiles >= 2 * 152) return {3, 128, 2};
+  if (npts > 16 && (npts + 63) / 64 * tiles >= 152) return {2, 64, 2};
+  if (npts > 8) return {1, 16, 5};
+  return {0, 8, 6};
+}
+// Row groups (CTAs of a chain group): one a tile for small data sets, else `want` (0: fill the chip once), so
+// that every group has the same number of tiles where that can be.
+inline int logreg_fp32_row_groups(int64_t n, int npts, int want) {
+  const LogregShape s = logreg_fp32_shape(n, npts);
+  const int64_t tiles = (n + 63) / 64;
+  if (tiles <= LR_ORDERED) return (int)(want > 0 ? std::min<int64_t>(want, tiles) : tiles);
+  const int cgroups = (npts + s.ct - 1) / s.ct;
+  const int64_t rg = std::min<int64_t>(want > 0 ? want : std::max(1, s.per_sm * 152 / cgroups), tiles);
+  const int64_t per = (tiles + rg - 1) / rg;
+  return (int)((tiles + per - 1) / per);
+}
+
+template <int CT, int NTH, int RG, int CG, int FG, int NB32, int NB64, int MINB>
+static cudaError_t logreg_fp32_launch_variant(const LogregArgs& A, int row_groups, bool attr, cudaStream_t st) {
+  const int dp = (A.p + 3) / 4 * 4;
+  const dim3 grid((A.npts + CT - 1) / CT, row_groups);
+  if (attr) {  // the shared-memory limit, at the most features each instance takes
+    cudaError_t e = cudaFuncSetAttribute(logreg_fp32_kernel<CT, NTH, RG, CG, FG, 32, NB32, MINB>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)LogregTile<CT, NTH, RG, CG, FG, 32, NB32>::bytes(32));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(logreg_fp32_kernel<CT, NTH, RG, CG, FG, 64, NB64, MINB>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)LogregTile<CT, NTH, RG, CG, FG, 64, NB64>::bytes(64));
+    return e;
+  }
+  if (dp <= 32)
+    logreg_fp32_kernel<CT, NTH, RG, CG, FG, 32, NB32, MINB>
+        <<<grid, NTH, LogregTile<CT, NTH, RG, CG, FG, 32, NB32>::bytes(dp), st>>>(A);
+  else
+    logreg_fp32_kernel<CT, NTH, RG, CG, FG, 64, NB64, MINB>
+        <<<grid, NTH, LogregTile<CT, NTH, RG, CG, FG, 64, NB64>::bytes(dp), st>>>(A);
+  return cudaGetLastError();
+}
+
+// variant < 0: sets every variant's shared-memory limit on the current device
+static cudaError_t logreg_fp32_launch(int variant, const LogregArgs& A, int row_groups, cudaStream_t st) {
+  const bool attr = variant < 0;
+  cudaError_t e = cudaSuccess;
+  if (attr || variant == 0) e = logreg_fp32_launch_variant<8, 32, 1, 1, 1, 2, 2, 6>(A, row_groups, attr, st);
+  if ((attr && e == cudaSuccess) || variant == 1)
+    e = logreg_fp32_launch_variant<16, 64, 1, 1, 1, 2, 2, 5>(A, row_groups, attr, st);
+  if ((attr && e == cudaSuccess) || variant == 2)
+    e = logreg_fp32_launch_variant<64, 256, 1, 1, 1, 2, 2, 2>(A, row_groups, attr, st);
+  if ((attr && e == cudaSuccess) || variant == 3)
+    e = logreg_fp32_launch_variant<128, 256, 1, 2, 1, 2, 2, 2>(A, row_groups, attr, st);
+  return e;
+}
+
+}  // namespace gbn

@@ -26,6 +26,7 @@
 #include "internal.h"
 #include "hs_finish.cuh"
 #include "lr_finish.cuh"
+#include "logreg_fp32.cuh"
 #include "sv_potential.cuh"
 
 namespace gbn {
@@ -53,134 +54,9 @@ __global__ void __launch_bounds__(512) hier_nc_kernel(const float* __restrict__ 
                          inv_ts, lane);
 }
 
-// ============================================================ logistic regression (FP32 SIMT)
-// Fused per row tile: logits = X_tile B^T -> (sigmoid, softplus) -> grad += E^T X_tile.
-constexpr int LR_RT = 64;  // rows per tile
-constexpr int LR_CT = 64;  // chains per CTA
-
-__global__ void __launch_bounds__(256) logreg_simt_kernel(const float* __restrict__ X, const float* __restrict__ y,
-                                                          int64_t N, int p, int DP, const float* __restrict__ Q,
-                                                          int npts, int ld, float* __restrict__ part_g,
-                                                          double* __restrict__ part_ll, int row_groups,
-                                                          const int32_t* pending) {
-  if (pending && *pending == 0) return;
-  extern __shared__ __align__(16) float smem[];
-  float* XsT = smem;                // [DP][RT]
-  float* Xs = XsT + DP * LR_RT;     // [RT][DP]
-  float* BsT = Xs + LR_RT * DP;     // [DP][CT]
-  float* Es = BsT + DP * LR_CT;     // [RT][CT]
-  float* ys = Es + LR_RT * LR_CT;   // [RT]
-  double* red = (double*)(ys + LR_RT);  // [16][CT]
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int c0 = blockIdx.x * LR_CT;
-  const int rg = blockIdx.y;
-  // chain coefficients, transposed
-  for (int k = tid; k < DP * LR_CT; k += 256) {
-    int cc = k / DP, d = k % DP;
-    float v = 0.0f;
-    if (d < p && c0 + cc < npts) v = Q[(size_t)(c0 + cc) * ld + d];
-    BsT[d * LR_CT + cc] = v;
-  }
-  const int cg = tid & 15, dg = tid >> 4;  // phase-3 mapping
-  const bool g_active = dg * 4 < DP;
-  float gacc[4][4];
-  double llacc[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    llacc[i] = 0.0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) gacc[i][j] = 0.0f;
-  }
-  int64_t ntiles = (N + LR_RT - 1) / LR_RT;
-  for (int64_t tile = rg; tile < ntiles; tile += row_groups) {
-    int64_t r0 = tile * LR_RT;
-    __syncthreads();
-    for (int k = tid; k < LR_RT * DP; k += 256) {
-      int r = k / DP, d = k % DP;
-      float v = 0.0f;
-      if (d < p && r0 + r < N) v = X[(r0 + r) * (int64_t)p + d];
-      Xs[r * DP + d] = v;
-      XsT[d * LR_RT + r] = v;
-    }
-    if (tid < LR_RT) ys[tid] = (r0 + tid < N) ? y[r0 + tid] : 0.0f;
-    __syncthreads();
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-    for (int d = 0; d < DP; ++d) {
-      float4 xv = *reinterpret_cast<const float4*>(&XsT[d * LR_RT + ty * 4]);
-      float4 bv = *reinterpret_cast<const float4*>(&BsT[d * LR_CT + tx * 4]);
-      float xa[4] = {xv.x, xv.y, xv.z, xv.w};
-      float ba[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xa[i], ba[j], acc[i][j]);
-    }
-    float llt[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // this tile's 4 rows, folded into FP64 once per tile
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int r = ty * 4 + i;
-      bool rv = (r0 + r) < N;
-      float yy = ys[r];
-      float ev[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float l = acc[i][j];
-        float t = expf(-fabsf(l));
-        float sp = fmaxf(l, 0.0f) + log1pf(t);
-        float inv = 1.0f / (1.0f + t);
-        float sig = (l >= 0.0f) ? inv : t * inv;
-        bool v = rv && (c0 + tx * 4 + j) < npts;
-        ev[j] = v ? (sig - yy) : 0.0f;
-        llt[j] += v ? (sp - yy * l) : 0.0f;
-      }
-      *reinterpret_cast<float4*>(&Es[r * LR_CT + tx * 4]) = make_float4(ev[0], ev[1], ev[2], ev[3]);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) llacc[j] += (double)llt[j];
-    __syncthreads();
-    if (g_active) {
-      for (int r = 0; r < LR_RT; ++r) {
-        float4 e4 = *reinterpret_cast<const float4*>(&Es[r * LR_CT + cg * 4]);
-        float4 x4 = *reinterpret_cast<const float4*>(&Xs[r * DP + dg * 4]);
-        float ea[4] = {e4.x, e4.y, e4.z, e4.w};
-        float xa[4] = {x4.x, x4.y, x4.z, x4.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) gacc[i][j] = fmaf(ea[i], xa[j], gacc[i][j]);
-      }
-    }
-  }
-  // partial gradient [rg][chain][64]
-  if (g_active) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int cc = c0 + cg * 4 + i;
-      if (cc < npts) {
-        float* dst = part_g + ((size_t)rg * npts + cc) * 64 + dg * 4;
-        *reinterpret_cast<float4*>(dst) = make_float4(gacc[i][0], gacc[i][1], gacc[i][2], gacc[i][3]);
-      }
-    }
-  }
-  // log-likelihood partials: reduce over ty
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 4; ++j) red[ty * LR_CT + tx * 4 + j] = llacc[j];
-  __syncthreads();
-  if (tid < LR_CT) {
-    double s = 0.0;
-    for (int k = 0; k < 16; ++k) s += red[k * LR_CT + tid];
-    if (c0 + tid < npts) part_ll[(size_t)rg * npts + c0 + tid] = s;
-  }
-}
-
-// sum partials, add the N(0, scale) prior; warp per point
-// lin (optional, FP64 [p]): a linear term lin . b of the log-likelihood computed outside the kernel
+// ============================================================ logistic regression
+// sum the tensor-core kernel's partials, add the N(0, scale) prior; warp per point
+// lin (FP64 [p]): a linear term lin . b of the log-likelihood computed outside the kernel
 __global__ void logreg_finish_kernel(const float* __restrict__ Q, int npts, int ld, int p, int row_groups,
                                      const float* __restrict__ part_g, const double* __restrict__ part_ll,
                                      const double* __restrict__ lin, float inv_var_f, double pe_const,
@@ -377,21 +253,18 @@ __global__ void scale_rows_kernel(const double* __restrict__ cot, float* __restr
 }
 
 // ============================================================ host side
-static int logreg_dp(int p) { return ((p + 3) / 4) * 4; }
-
 cudaError_t ensure_potential_scratch(ModelDev& m, int points) {
   if (points <= m.scratch_points) return cudaSuccess;
   free_potential_scratch(m);
   cudaError_t e = cudaSuccess;
   if (m.family == 2) {
-    // row groups: enough CTAs for ~4 waves over 152 SMs; buffers hold twice that for the tuner
-    int cgroups = (points + LR_CT - 1) / LR_CT;
-    int64_t ntiles = (m.n + LR_RT - 1) / LR_RT;
-    int rg = (int)((4 * 152 + cgroups - 1) / cgroups);
-    if (rg < 1) rg = 1;
-    if (rg > ntiles) rg = (int)ntiles;
-    m.row_groups = rg;
-    m.row_groups_cap = (int)std::min<int64_t>(2 * (int64_t)rg, ntiles);
+    // Partials for the row groups of both kernels: the tensor-core one takes at most 152 over its blocks of
+    // 128 chains, the FP32 one its default, with room for the tuner to try twice as many.
+    const int64_t ntiles = (m.n + 63) / 64;
+    const int tc_rg = (int)std::min<int64_t>(std::max(1, 152 / ((points + 127) / 128)), ntiles);
+    const int rg = logreg_fp32_row_groups(m.n, points, 0);
+    m.row_groups = std::max(tc_rg, rg);
+    m.row_groups_cap = (int)std::min<int64_t>(std::max<int64_t>(m.row_groups, 2 * (int64_t)rg), ntiles);
     if (m.tune.lr_rg > m.row_groups_cap) m.tune.lr_rg = 0;
     e = cudaMalloc(&m.part_g, sizeof(float) * (size_t)m.row_groups_cap * points * 64);
     if (e == cudaSuccess) e = cudaMalloc(&m.part_ll, sizeof(double) * (size_t)m.row_groups_cap * points);
@@ -426,19 +299,14 @@ void free_potential_scratch(ModelDev& m) {
   m.scratch_points = 0;
 }
 
-static size_t logreg_smem(int DP) {
-  return sizeof(float) * (size_t)(DP * LR_RT + LR_RT * DP + DP * LR_CT + LR_RT * LR_CT + LR_RT) +
-         sizeof(double) * 16 * LR_CT;
-}
-
 namespace {
 std::mutex g_simt_attr_mu;
 std::vector<char> g_simt_attr_done;  // per device ordinal: the shared-memory limit is raised
 }  // namespace
 
-// logreg_simt_kernel needs about 74 KB of dynamic shared memory at 64 features, above the 48 KB
-// default.  The limit is a per-device attribute of the kernel, so it is raised once for every
-// device the kernel runs on (with that device current), under a mutex.
+// The FP32 logistic kernels need up to 104 KB of dynamic shared memory, above the 48 KB default.  The
+// limit is a per-device attribute of a kernel, so it is raised once for every device they run on (with
+// that device current), under a mutex.
 cudaError_t logreg_simt_smem_attr() {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -447,9 +315,27 @@ cudaError_t logreg_simt_smem_attr() {
   std::lock_guard<std::mutex> lock(g_simt_attr_mu);
   if ((int)g_simt_attr_done.size() <= dev) g_simt_attr_done.resize((size_t)dev + 1, 0);
   if (g_simt_attr_done[(size_t)dev]) return cudaSuccess;
-  e = cudaFuncSetAttribute(logreg_simt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)logreg_smem(64));
+  LogregArgs probe{};
+  probe.p = 1;
+  probe.npts = 1;
+  e = logreg_fp32_launch(-1, probe, 1, 0);
   if (e == cudaSuccess) g_simt_attr_done[(size_t)dev] = 1;
   return e;
+}
+
+static cudaError_t launch_logreg_fp32(const float* x, const float* y, int64_t n, int p, double prior_scale,
+                                      const float* Q, int npts, int ld, int row_groups, float* part_g, double* part_ll,
+                                      double* PE, float* G, const int32_t* pending, cudaStream_t st) {
+  cudaError_t e = logreg_simt_smem_attr();
+  if (e != cudaSuccess) return e;
+  const LogregArgs A{x, y, n, p, Q, npts, ld, part_g, part_ll, pending};
+  e = logreg_fp32_launch(logreg_fp32_shape(n, npts).variant, A, row_groups, st);
+  if (e != cudaSuccess) return e;  // checked per launch, so the first failing launch is the one reported
+  float ivf;
+  double pec;
+  logreg_prior_consts(prior_scale, p, &ivf, &pec);
+  logreg_fp32_finish_kernel<<<npts, 256, 0, st>>>(A, row_groups, ivf, pec, PE, G);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, float* G, const int32_t* pending,
@@ -469,19 +355,12 @@ cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, 
       break;
     case 2: {
       if (m.precision == 1 && m.tc) return logreg_tc_launch(m, Q, npts, PE, G, pending, st, fused_tick);
-      int DP = logreg_dp(m.p);
-      size_t sm = logreg_smem(DP);
-      e = logreg_simt_smem_attr();
+      // the tuned row groups belong to the handle's own number of points; the partials bound any other
+      const int want = npts == m.scratch_points ? m.tune.lr_rg : 0;
+      const int rg = (int)std::min<int64_t>(logreg_fp32_row_groups(m.n, npts, want),
+                                            (int64_t)m.row_groups_cap * m.scratch_points / npts);
+      e = launch_logreg_fp32(m.x, m.y, m.n, m.p, m.hyper[0], Q, npts, ld, rg, m.part_g, m.part_ll, PE, G, pending, st);
       if (e != cudaSuccess) return e;
-      const int rg = m.tune.lr_rg > 0 ? m.tune.lr_rg : m.row_groups;
-      dim3 grid((npts + LR_CT - 1) / LR_CT, rg);
-      logreg_simt_kernel<<<grid, 256, sm, st>>>(m.x, m.y, m.n, m.p, DP, Q, npts, ld, m.part_g, m.part_ll, rg,
-                                                pending);
-      float ivf;
-      double pec;
-      logreg_prior_consts(m.hyper[0], m.p, &ivf, &pec);
-      logreg_finish_kernel<<<(npts + 7) / 8, 256, 0, st>>>(Q, npts, ld, m.p, rg, m.part_g, m.part_ll, nullptr, ivf,
-                                                           pec, PE, G, pending);
       break;
     }
     case 3: {
@@ -594,9 +473,15 @@ cudaError_t autotune_potential(ModelDev& m, const float* Q, int npts, double* PE
         cand.push_back(t);
       }
     } else if (m.family == 2 && !(m.precision == 1 && m.tc)) {
-      for (int rg : {std::max(1, m.row_groups / 2), m.row_groups, m.row_groups_cap}) {
-        t.lr_rg = rg;
+      const int rg0 = logreg_fp32_row_groups(m.n, npts, 0);
+      if (m.n <= 64 * LR_ORDERED) {  // one row group a tile
+        t.lr_rg = rg0;
         cand.push_back(t);
+      } else {
+        for (int rg : {std::max(1, rg0 / 2), rg0, std::min(2 * rg0, m.row_groups_cap)}) {
+          t.lr_rg = logreg_fp32_row_groups(m.n, npts, rg);
+          cand.push_back(t);
+        }
       }
     } else if (m.family == 3) {
       for (int tm : {2, 4})
@@ -713,20 +598,8 @@ namespace gbn {
 cudaError_t launch_logreg_simt_scratch(const float* x, const float* y, int64_t n, int p, double prior_scale,
                                        const float* Q, int npts, int row_groups, float* part_g, double* part_ll,
                                        double* PE, float* G, cudaStream_t st) {
-  cudaError_t e = logreg_simt_smem_attr();
-  if (e != cudaSuccess) return e;
-  int DP = logreg_dp(p);
-  dim3 grid((npts + LR_CT - 1) / LR_CT, row_groups);
-  logreg_simt_kernel<<<grid, 256, logreg_smem(DP), st>>>(x, y, n, p, DP, Q, npts, p, part_g, part_ll, row_groups,
-                                                         nullptr);
-  e = cudaGetLastError();  // checked per launch, so the first failing launch is the one reported
-  if (e != cudaSuccess) return e;
-  float ivf;
-  double pec;
-  logreg_prior_consts(prior_scale, p, &ivf, &pec);
-  logreg_finish_kernel<<<(npts + 7) / 8, 256, 0, st>>>(Q, npts, p, p, row_groups, part_g, part_ll, nullptr, ivf, pec,
-                                                       PE, G, nullptr);
-  return cudaGetLastError();
+  return launch_logreg_fp32(x, y, n, p, prior_scale, Q, npts, p, logreg_fp32_row_groups(n, npts, row_groups), part_g,
+                            part_ll, PE, G, nullptr, st);
 }
 
 void horseshoe_finish_launch(const float* Q, int npts, int ld, int P, int64_t N, const float* part_gb, int splits,
