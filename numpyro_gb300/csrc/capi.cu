@@ -744,7 +744,8 @@ int gbn_run(gbn_handle h, void* stream, gbn_state* st, int32_t num_iterations, i
     if (e != cudaSuccess) return cuda_fail(h, e, "gbn_run: queue");
     if (h->m.family == GBN_FAMILY_SV) {
       SvView sv{h->m.y, (int)h->m.n, h->m.hyper[2] != 0.0, h->m.hyper[0], h->m.hyper[1]};
-      launch_persistent_sv(h->dP, sv, h->counters + 7, h->C, h->D, s);
+      launch_persistent_sv(h->dP, sv, h->counters + 7, h->C, h->D, h->cfg.algo == GBN_ALGO_NUTS,
+                           h->cfg.find_heuristic_step_size && h->cfg.adapt_step_size && h->num_warmup > 0, s);
     } else {
       HierView hv{h->m.y, h->m.hier_sinv, h->m.hier_cmodel, h->m.offsets, h->m.chains_per_model, h->m.num_models,
                   (float)(1.0 / (h->m.hyper[0] * h->m.hyper[0])), (float)(1.0 / h->m.hyper[1])};
@@ -842,7 +843,8 @@ int gbn_sample_async(gbn_handle h, void* stream, gbn_state* st) {
   if (h->persistent) {
     if (h->m.family == GBN_FAMILY_SV) {
       SvView sv{h->m.y, (int)h->m.n, h->m.hyper[2] != 0.0, h->m.hyper[0], h->m.hyper[1]};
-      launch_persistent_sv(h->dP, sv, h->counters + 7, h->C, h->D, s);
+      launch_persistent_sv(h->dP, sv, h->counters + 7, h->C, h->D, h->cfg.algo == GBN_ALGO_NUTS,
+                           h->cfg.find_heuristic_step_size && h->cfg.adapt_step_size && h->num_warmup > 0, s);
     } else {
       HierView hv{h->m.y, h->m.hier_sinv, h->m.hier_cmodel, h->m.offsets, h->m.chains_per_model, h->m.num_models,
                   (float)(1.0 / (h->m.hyper[0] * h->m.hyper[0])), (float)(1.0 / h->m.hyper[1])};

@@ -145,6 +145,14 @@ struct Comp32 {
     c += (s - (t - bp)) + (x - bp);
     s = t;
   }
+  // add(a * b) with the product exact inside fused multiply-adds: said outright, so that every kernel that
+  // inlines it gives the same bits
+  __device__ __forceinline__ void add_fused(float a, float b) {
+    const float t = fmaf(a, b, s);
+    const float bp = t - s;
+    c += (s - (t - bp)) + fmaf(a, b, -bp);
+    s = t;
+  }
   __device__ __forceinline__ float value() const { return s + c; }
 };
 

@@ -51,8 +51,8 @@ constexpr float FLT32_MAX = 3.40282347e+38f;
 // The factorisation runs in FP64 in place (U in the upper triangle, S below the diagonal); A is
 // zeroed afterwards (it is the Welford m2 buffer, reset at every window end).  One group per
 // matrix; threads own columns.
-template <int NT>
-__device__ void dense_factor(const Group<NT>& g, double* A, int D, int ld, float* inv, float* sq, float* sqi) {
+template <int NT, class Threads>
+__device__ void dense_factor(const Threads& g, double* A, int D, int ld, float* inv, float* sq, float* sqi) {
   for (int j = g.tid; j < D; j += NT)
     for (int i = 0; i < D; ++i) inv[(size_t)i * ld + j] = (float)A[(size_t)i * ld + j];
   for (int k = D - 1; k >= 0; --k) {
@@ -88,10 +88,10 @@ __device__ void dense_factor(const Group<NT>& g, double* A, int D, int ld, float
   g.sync();
 }
 
-template <int NT, bool DM = false>  // DM: dense mass matrices
+template <int NT, bool DM = false, class Threads = Group<NT>>  // DM: dense mass matrices
 struct Chain {
   const AdvParams& P;
-  Group<NT> g;
+  Threads g;
   double* red;
   int c;   // chain index
   int D;   // this chain's latent dim
@@ -662,7 +662,7 @@ struct Chain {
             const bool keep = !blk || i == j || (blk[i] >= 0 && blk[i] == blk[j]);
             m2[o] = keep ? a * (m2[o] * inv_nm1) + (i == j ? shrink : 0.0) : 0.0;
           }
-        dense_factor(g, m2, D, ld, MX(P.s.inverse_mass_matrix), MX(P.s.mass_matrix_sqrt),
+        dense_factor<NT>(g, m2, D, ld, MX(P.s.inverse_mass_matrix), MX(P.s.mass_matrix_sqrt),
                      MX(P.s.mass_matrix_sqrt_inv));
         for (int d = g.tid; d < D; d += NT) mean[d] = 0.0;
         if (g.tid == 0) P.s.mm_n[c] = 0;
@@ -971,6 +971,7 @@ __device__ __forceinline__ const AdvParams& stage_params(const AdvParams* __rest
 }  // namespace gbn
 
 #include "hier_engine.cuh"
+#include "sv_engine.cuh"
 
 namespace gbn {
 
@@ -1134,7 +1135,7 @@ __global__ void init_dense_mass_kernel(const AdvParams* __restrict__ Pp, const f
     A[o] = (inv_mass_init && i < Dc && j < Dc) ? (double)inv_mass_init[base + o] : 0.0;
   }
   __syncwarp();
-  if (inv_mass_init) dense_factor(Group<32>{lane}, A, Dc, ld, inv, sq, sqi);
+  if (inv_mass_init) dense_factor<32>(Group<32>{lane}, A, Dc, ld, inv, sq, sqi);
 }
 
 __global__ void set_phase_kernel(const AdvParams* __restrict__ Pp, int phase, int iters) {
@@ -1301,12 +1302,53 @@ void launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* qu
     persistent_hier_kernel<false><<<blocks, 256, 0, st>>>(dP, hv, queue_head, order);
 }
 
-void launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D,
+template <int K, bool NC>
+static void launch_sv_reg(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, int sms,
                           cudaStream_t st) {
+  const size_t smem = sv_engine_smem(D, NC, K);
+  cudaFuncSetAttribute(persistent_sv_reg_kernel<K, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int blocks = C;
+  if (C > sms) {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_sv_reg_kernel<K, NC>, 320, smem);
+    blocks = std::min(C, sms * std::max(per_sm, 1));
+  }
+  persistent_sv_reg_kernel<K, NC><<<blocks, 320, smem, st>>>(dP, sv, queue_head);
+}
+template <int K>
+static void launch_sv_reg(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, int sms,
+                          cudaStream_t st) {
+  if (sv.noncentred)
+    launch_sv_reg<K, true>(dP, sv, queue_head, C, D, sms, st);
+  else
+    launch_sv_reg<K, false>(dP, sv, queue_head, C, D, sms, st);
+}
+
+void launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, bool nuts,
+                          bool searches, cudaStream_t st) {
   int dev = 0, sms = 0, per_sm = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  // The on-chip engine holds 17 coordinates a thread (4,352); HMC, longer walks and warmup with step-size
+  // searches run the state machine over memory.
+  if (nuts && !searches && D <= 4352 && (!sv.noncentred || sv.T <= 4096)) {
+    if (D <= 256)
+      launch_sv_reg<1>(dP, sv, queue_head, C, D, sms, st);
+    else if (D <= 512)
+      launch_sv_reg<2>(dP, sv, queue_head, C, D, sms, st);
+    else if (D <= 1024)
+      launch_sv_reg<4>(dP, sv, queue_head, C, D, sms, st);
+    else if (D <= 1536)
+      launch_sv_reg<6>(dP, sv, queue_head, C, D, sms, st);
+    else if (D <= 2304)
+      launch_sv_reg<9>(dP, sv, queue_head, C, D, sms, st);
+    else if (D <= 3328)
+      launch_sv_reg<13>(dP, sv, queue_head, C, D, sms, st);
+    else
+      launch_sv_reg<17>(dP, sv, queue_head, C, D, sms, st);
+    return;
+  }
   // On-chip rows make each leaf about a quarter faster (T = 4096 on GB300), but at 12 D floats per
   // CTA they can cost resident chains (197 KB: one CTA per SM, against two with global rows).  They
   // are used only when every chain is resident either way.

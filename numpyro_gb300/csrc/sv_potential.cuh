@@ -78,6 +78,65 @@ __device__ __forceinline__ float sv_grad_lnu(double S_l1p, double S_frac, double
   return (float)(-(dnu * nu + 1.0));
 }
 
+// One step of the centred walk: accumulates the sums and returns dU/dh_t.
+__device__ __forceinline__ float sv_centred_step(int t, int T, float h, float hp, float hn, float rt, float nuf,
+                                                 float inv_nuf, float inv_s2, Comp32& sdd, Comp32& sl1p,
+                                                 Comp32& sfrac, Comp32& sh) {
+  const float dprev = (t == 0) ? h : h - hp;
+  const float dnext = (t + 1 < T) ? hn - h : 0.0f;
+  const float yv = rt * expf(-h);
+  const float y2 = yv * yv;
+  const float q = y2 * inv_nuf;
+  const float frac = __fdividef(y2, nuf + y2);
+  sdd.add_fused(dprev, dprev);
+  sl1p.add(log1pf(q));
+  sfrac.add(frac);
+  sh.add(h);
+  return (dprev - dnext) * inv_s2 + 1.0f - (nuf + 1.0f) * frac;
+}
+
+// One step of the non-centred walk: extends it by e, accumulates, returns a_t = d log p(r_t | h_t) / d h_t.
+// in = false (with e = 0 and rt = 0): a step past the chunk, which adds zeros.
+struct SvNcSums {
+  Comp32 l1p, frac, h, as, e2, atot;
+};
+__device__ __forceinline__ float sv_nc_step(Comp32& S, float e, float rt, float sf, float nuf, float inv_nuf,
+                                            SvNcSums& a, bool in = true) {
+  S.add(e);
+  const float St = S.value();
+  const float h = in ? __fmul_rn(sf, St) : 0.0f;
+  const float yv = rt * expf(-h);
+  const float y2 = yv * yv;
+  const float frac = __fdividef(y2, nuf + y2);
+  const float at = in ? (nuf + 1.0f) * frac - 1.0f : 0.0f;
+  a.l1p.add(log1pf(y2 * inv_nuf));
+  a.frac.add(frac);
+  a.h.add(h);
+  a.as.add_fused(at, in ? St : 0.0f);
+  a.e2.add_fused(e, e);
+  a.atot.add(at);
+  return at;
+}
+
+// -U and dU/d log s from the sums; log_rates = log(s_rate) + log(nu_rate), lg0/lg1 = lgamma(nu / 2), lgamma((nu + 1) / 2)
+__device__ __forceinline__ double sv_log_joint(bool noncentred, double S_walk, double S_l1p, double S_h, double T,
+                                               double lnu, double ls, double nu, double s, double inv_s,
+                                               double log_rates, double s_rate, double nu_rate, double lg0, double lg1) {
+  double lp = log_rates - s_rate * s + ls - nu_rate * nu + lnu;
+  if (noncentred)
+    lp += -0.5 * S_walk - 0.5 * T * SV_LOG_2PI;
+  else
+    lp += -0.5 * S_walk * (inv_s * inv_s) - T * ls - 0.5 * T * SV_LOG_2PI;
+  const double zc = 0.5 * lnu + 0.5 * SV_LOG_PI + lg0 - lg1;
+  return lp + (-0.5 * (nu + 1.0) * S_l1p - S_h - T * zc);
+}
+__device__ __forceinline__ float sv_grad_ls(bool noncentred, double S_dd_or_as, double T, double s, double inv_s,
+                                            double s_rate) {
+  if (noncentred) return (float)(-s * S_dd_or_as + s_rate * s - 1.0);
+  const double ds = S_dd_or_as * (inv_s * inv_s * inv_s) - T * inv_s - s_rate;
+  return (float)(-(ds * s + 1.0));
+}
+
 // The potentials are compiled out of line: the tick and persistent kernels then run one and
 // the same instruction sequence (inlined into different kernels, floating-point contraction
 // could differ between them and break their bit-identity).
@@ -109,34 +168,18 @@ __device__ __noinline__ void sv_potential_block(const float* z, float* g, double
     for (int k = 0; k < U; ++k) {
       const int t = t0 + k * NT;
       if (t >= T) continue;
-      const float h = hv[k];
-      const float dprev = (t == 0) ? h : h - hp[k];
-      const float dnext = (t + 1 < T) ? hn[k] - h : 0.0f;
-      const float yv = rv[k] * expf(-h);
-      const float y2 = yv * yv;
-      const float q = y2 * inv_nuf;
-      const float frac = __fdividef(y2, nuf + y2);
-      sdd.add(dprev * dprev);
-      sl1p.add(log1pf(q));
-      sfrac.add(frac);
-      sh.add(h);
-      g[t] = (dprev - dnext) * inv_s2 + 1.0f - (nuf + 1.0f) * frac;
+      g[t] = sv_centred_step(t, T, hv[k], hp[k], hn[k], rv[k], nuf, inv_nuf, inv_s2, sdd, sl1p, sfrac, sh);
     }
   }
   FF f_dd = comp_ff(sdd), f_l1p = comp_ff(sl1p), f_frac = comp_ff(sfrac), f_h = comp_ff(sh);
   grp.sum2ff(f_dd, f_l1p, sm.red);
   grp.sum2ff(f_frac, f_h, sm.red);
   if (tid == 0) {
-    const double lnu = lnuf, ls = lsf, nu = sm.special[4], s = sm.special[6], inv_s = sm.special[7];
-    double S_dd = ff_value(f_dd), S_l1p = ff_value(f_l1p), S_frac = ff_value(f_frac), S_h = ff_value(f_h);
-    double lp = sm.special[8] - s_rate * s + ls - nu_rate * nu + lnu;
-    lp += -0.5 * S_dd * (inv_s * inv_s) - (double)T * ls - 0.5 * (double)T * SV_LOG_2PI;
-    double zc = 0.5 * lnu + 0.5 * SV_LOG_PI + sm.special[0] - sm.special[1];
-    lp += -0.5 * (nu + 1.0) * S_l1p - S_h - (double)T * zc;
-    *pe_out = -lp;
-    g[T] = sv_grad_lnu(S_l1p, S_frac, (double)T, nu_rate, sm.special);
-    double ds = S_dd * (inv_s * inv_s * inv_s) - (double)T * inv_s - s_rate;
-    g[T + 1] = (float)(-(ds * s + 1.0));
+    const double s = sm.special[6], inv_s = sm.special[7], S_dd = ff_value(f_dd), S_l1p = ff_value(f_l1p);
+    *pe_out = -sv_log_joint(false, S_dd, S_l1p, ff_value(f_h), (double)T, lnuf, lsf, sm.special[4], s, inv_s,
+                            sm.special[8], s_rate, nu_rate, sm.special[0], sm.special[1]);
+    g[T] = sv_grad_lnu(S_l1p, ff_value(f_frac), (double)T, nu_rate, sm.special);
+    g[T + 1] = sv_grad_ls(false, S_dd, (double)T, s, inv_s, s_rate);
   }
 }
 
@@ -195,25 +238,9 @@ __device__ __noinline__ void sv_nc_potential_block(const float* z, float* g, dou
   sv_special_functions<NT>(lnuf, lsf, s_rate, nu_rate, tid, sm.special);
   const int chunk = (T + NT - 1) / NT;
   const int t0 = min(T, tid * chunk), t1 = min(T, t0 + chunk);
-  Comp32 sl1p{0.0f, 0.0f}, sfrac{0.0f, 0.0f}, sh{0.0f, 0.0f}, sas{0.0f, 0.0f}, se2{0.0f, 0.0f},
-      atot{0.0f, 0.0f};
+  SvNcSums a{};
   // one step of the forward pass: extend the walk, accumulate, return a_t
-  auto forward_step = [&](Comp32& S, float e, float r) -> float {
-    S.add(e);
-    const float St = S.value();
-    const float h = sf * St;
-    const float yv = r * expf(-h);
-    const float y2 = yv * yv;
-    const float frac = __fdividef(y2, nuf + y2);
-    const float at = (nuf + 1.0f) * frac - 1.0f;  // d log p(r_t | h_t) / d h_t
-    sl1p.add(log1pf(y2 * inv_nuf));
-    sfrac.add(frac);
-    sh.add(h);
-    sas.add(at * St);
-    se2.add(e * e);
-    atot.add(at);
-    return at;
-  };
+  auto forward_step = [&](Comp32& S, float e, float r) -> float { return sv_nc_step(S, e, r, sf, nuf, inv_nuf, a); };
   if (chunk <= SV_REG_CHUNK) {
     // the chunk's h_base, returns and a_t stay in registers between the passes
     float ev[SV_REG_CHUNK], rv[SV_REG_CHUNK], av[SV_REG_CHUNK];
@@ -233,7 +260,7 @@ __device__ __noinline__ void sv_nc_potential_block(const float* z, float* g, dou
 #pragma unroll
     for (int i = 0; i < SV_REG_CHUNK; ++i) av[i] = (t0 + i < t1) ? forward_step(S, ev[i], rv[i]) : 0.0f;
     // reverse pass: suffix sums of a_t from the thread's starting suffix
-    const FF suf = block_excl_rscan<NT>(comp_ff(atot), tid, sm.warp_tot[1]);
+    const FF suf = block_excl_rscan<NT>(comp_ff(a.atot), tid, sm.warp_tot[1]);
     Comp32 A{suf.hi, suf.lo};
 #pragma unroll
     for (int i = SV_REG_CHUNK - 1; i >= 0; --i) {
@@ -248,28 +275,23 @@ __device__ __noinline__ void sv_nc_potential_block(const float* z, float* g, dou
     const FF ck = block_excl_scan<NT>(comp_ff(tot), tid, sm.warp_tot[0]);
     Comp32 S{ck.hi, ck.lo};
     for (int t = t0; t < t1; ++t) g[t] = forward_step(S, z[t], ret[t]);
-    const FF suf = block_excl_rscan<NT>(comp_ff(atot), tid, sm.warp_tot[1]);
+    const FF suf = block_excl_rscan<NT>(comp_ff(a.atot), tid, sm.warp_tot[1]);
     Comp32 A{suf.hi, suf.lo};
     for (int t = t1 - 1; t >= t0; --t) {
       A.add(g[t]);
       g[t] = z[t] - sf * A.value();
     }
   }
-  FF f_l1p = comp_ff(sl1p), f_frac = comp_ff(sfrac), f_h = comp_ff(sh), f_as = comp_ff(sas);
+  FF f_l1p = comp_ff(a.l1p), f_frac = comp_ff(a.frac), f_h = comp_ff(a.h), f_as = comp_ff(a.as);
   grp.sum2ff(f_l1p, f_frac, sm.red);
   grp.sum2ff(f_h, f_as, sm.red);
-  const FF f_e2 = grp.sumff(comp_ff(se2), sm.red);
+  const FF f_e2 = grp.sumff(comp_ff(a.e2), sm.red);
   if (tid == 0) {
-    const double lnu = lnuf, ls = lsf, nu = sm.special[4], s = sm.special[6];
-    double S_l1p = ff_value(f_l1p), S_frac = ff_value(f_frac), S_h = ff_value(f_h), S_as = ff_value(f_as),
-           S_e2 = ff_value(f_e2);
-    double lp = sm.special[8] - s_rate * s + ls - nu_rate * nu + lnu;
-    lp += -0.5 * S_e2 - 0.5 * (double)T * SV_LOG_2PI;
-    double zc = 0.5 * lnu + 0.5 * SV_LOG_PI + sm.special[0] - sm.special[1];
-    lp += -0.5 * (nu + 1.0) * S_l1p - S_h - (double)T * zc;
-    *pe_out = -lp;
-    g[T] = sv_grad_lnu(S_l1p, S_frac, (double)T, nu_rate, sm.special);
-    g[T + 1] = (float)(-s * S_as + s_rate * s - 1.0);
+    const double s = sm.special[6], S_l1p = ff_value(f_l1p);
+    *pe_out = -sv_log_joint(true, ff_value(f_e2), S_l1p, ff_value(f_h), (double)T, lnuf, lsf, sm.special[4], s, 0.0,
+                            sm.special[8], s_rate, nu_rate, sm.special[0], sm.special[1]);
+    g[T] = sv_grad_lnu(S_l1p, ff_value(f_frac), (double)T, nu_rate, sm.special);
+    g[T + 1] = sv_grad_ls(true, ff_value(f_as), (double)T, s, 0.0, s_rate);
   }
 }
 
