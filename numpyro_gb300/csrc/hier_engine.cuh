@@ -16,7 +16,9 @@
 // of the butterfly (ff_add commutes).  The uniforms of a transition's first 31 leaves come from one
 // Philox evaluation (a lane each).
 // Measured against the state machine over memory (persistent_hier_kernel): eight schools, 4 chains,
-// 200 transitions 10.3 -> 4.8 ms; 16,384 chains of 4 to 256 groups, 5 transitions 8.2 -> 4.2 ms a call.
+// 200 transitions 10.3 -> 4.8 ms; 16,384 chains of 4 to 256 groups, 5 transitions 8.2 -> 4.2 ms a call;
+// dense mass matrices (M^-1 in shared memory, one row broadcast by shuffle a step), 64 chains of 32 dimensions,
+// 100 warmup transitions 25.6 -> 9.4 ms, half of it from a warp per SM instead of eight.
 #pragma once
 
 namespace gbn {
@@ -90,10 +92,11 @@ __device__ __noinline__ float hier_momentum(Seed s, uint32_t chain, uint32_t n, 
 // The end of a transition (state, collection, adaptation and its step-size searches) through the
 // generic state machine, out of line: it runs once per tree and its registers stay out of the leaf
 // loop.  Returns how many transitions the chain has left.
+template <bool DM>
 __device__ __noinline__ int hier_end_transition(const AdvParams& P, const HierView& hv, int c, int m, int D, int lane,
                                                 double pe, double energy, int num_steps, double accept_prob,
                                                 int diverging, const float* znew, const float* gnew) {
-  Chain<32> ch{P, Group<32>{lane}, nullptr, c, D, P.D, P.e.ctl[c], nullptr};
+  Chain<32, DM> ch{P, Group<32>{lane}, nullptr, c, D, P.D, P.e.ctl[c], nullptr};
   __syncwarp();  // ctl read by every lane before lane 0 writes it back
   const size_t row = (size_t)c * P.D;
   if (ch.finish_transition(pe, energy, num_steps, accept_prob, diverging, znew, gnew)) {
@@ -114,9 +117,10 @@ __device__ __noinline__ int hier_end_transition(const AdvParams& P, const HierVi
 
 // Every transition of chain c, of latent dimension at most 32 K.  ck_warp: ck_floats floats of
 // shared memory for the shallowest (most used) of its U-turn checkpoints (momentum and momentum sum).
-template <int K>
+// DM: dense mass matrices; minv then holds 32 K floats of shared memory for each row of M^-1.
+template <int K, bool DM>
 __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierView& hv, int c, int m, int D, int lane,
-                                               float* ck_warp, int ck_floats) {
+                                               float* ck_warp, int ck_floats, float* minv) {
   const uint32_t FULL = 0xffffffffu;
   const int ck_slots = ck_floats / (64 * K);
   const int j0 = hv.off[m], J = hv.off[m + 1] - j0;
@@ -131,26 +135,74 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
   while (iters_left > 0) {
     // ---------------------------------------------------------- start of a transition
     const uint32_t n = P.s.rng_key[2 * c + 1], cid = P.s.rng_key[2 * c];
-    float z[K], r[K], g[K], mi[K], rss[K];
+    float z[K], r[K], g[K], mi[DM ? 1 : K], rss[K];
     float kin0f = 0.0f;
+    // v = M^-1 x, terms in the order of Chain::sym_matvec
+    auto matvec = [&](const float* x, float* v) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] = 0.0f;
+#pragma unroll
+      for (int kb = 0; kb < K; ++kb) {
+        const int rows = min(32, D - 32 * kb);
+#pragma unroll 8
+        for (int j = 0; j < rows; ++j) {
+          const float xj = __shfl_sync(FULL, x[kb], j);
+          const float* const a = minv + (32 * kb + j) * (32 * K) + lane;
+#pragma unroll
+          for (int k = 0; k < K; ++k) v[k] = fmaf(a[32 * k], xj, v[k]);
+        }
+      }
+    };
+    if (DM) {  // M^-1 may have changed at a window end
+      const float* const src = P.s.inverse_mass_matrix + row * P.D;
+      __syncwarp();
+      for (int j = 0; j < D; ++j)
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          minv[j * (32 * K) + 32 * k + lane] = lane + 32 * k < D ? src[(size_t)j * P.D + lane + 32 * k] : 0.0f;
+      __syncwarp();
+    }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int d = lane + 32 * k;
       const bool in = d < D;
       z[k] = in ? P.s.z[row + d] : 0.0f;
       g[k] = in ? P.s.z_grad[row + d] : 0.0f;
-      mi[k] = in ? P.s.inverse_mass_matrix[row + d] : 0.0f;
+      if (!DM) mi[DM ? 0 : k] = in ? P.s.inverse_mass_matrix[row + d] : 0.0f;
       r[k] = 0.0f;
       rss[k] = 0.0f;
       if (k < kc) {
         const float e = hier_momentum(P.seed, cid, n, d);
-        if (in) {
+        if (DM) {
+          if (in) P.e.tmp[row + d] = e;
+        } else if (in) {
           r[k] = P.s.mass_matrix_sqrt[row + d] * e;
-          kin0f = fmaf(mi[k] * r[k], r[k], kin0f);
+          kin0f = fmaf(mi[DM ? 0 : k] * r[k], r[k], kin0f);
           P.e.r_l[row + d] = r[k];
           P.e.rsum[row + d] = r[k];
         }
       }
+    }
+    if (DM) {  // r = S eps, as Chain::dense_momentum
+      __syncwarp();
+      const float* const eps = P.e.tmp + row;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int d = lane + 32 * k;
+        if (d < D) {
+          const float* const Si = P.s.mass_matrix_sqrt + (row + d) * P.D;
+          float acc = 0.0f;
+#pragma unroll 4
+          for (int j = 0; j < D; ++j) acc = fmaf(Si[j], eps[j], acc);
+          r[k] = acc;
+          P.e.r_l[row + d] = acc;
+          P.e.rsum[row + d] = acc;
+        }
+      }
+      float v[K];
+      matvec(r, v);
+#pragma unroll
+      for (int k = 0; k < K; ++k) kin0f = fmaf(v[k], r[k], kin0f);
     }
     FF kff = ff_from(kin0f);
 #pragma unroll
@@ -209,8 +261,14 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           const float rh = r[k] - 0.5f * eps * g[k];
-          z[k] = z[k] + eps * (mi[k] * rh);
+          if (!DM) z[k] = z[k] + eps * (mi[DM ? 0 : k] * rh);
           r[k] = rh;
+        }
+        float v[K];
+        if (DM) {
+          matvec(r, v);
+#pragma unroll
+          for (int k = 0; k < K; ++k) z[k] = z[k] + eps * v[k];
         }
         // ------------------------------------------------------ potential (hier_potential.cuh)
         // group j = lane + 32 k is element j + 2: two lanes up
@@ -256,8 +314,13 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
           const float rn = r[k] - 0.5f * eps * gn;
           r[k] = rn;
           g[k] = gn;
-          kinf = fmaf(mi[k] * rn, rn, kinf);
+          if (!DM) kinf = fmaf(mi[DM ? 0 : k] * rn, rn, kinf);
           rss[k] = leaf == 0 ? rn : rss[k] + rn;
+        }
+        if (DM) {
+          matvec(r, v);
+#pragma unroll
+          for (int k = 0; k < K; ++k) kinf = fmaf(v[k], r[k], kinf);
         }
         // ------------------------------------------------------ checkpoints and U-turn checks
         const int idx_max = __popc((unsigned)(leaf >> 1));
@@ -271,24 +334,39 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
           float* const rc = on_chip ? ck_warp + idx * (64 * K) : r_ck + idx * P.D;
           float* const rsc = on_chip ? rc + 32 * K : rs_ck + idx * P.D;
           float ax = odd ? 0.0f : 1.0f, ay = ax;  // 1: no turn
+          float left[K], mid[K];  // DM: the checkpoint's momentum, the subtree's sum less the end points' mean
 #pragma unroll
           for (int k = 0; k < K; ++k) {
             const int d = lane + 32 * k;
+            if (DM) left[k] = mid[k] = 0.0f;
             if (d >= D) continue;
             if (odd) {
               const float av = rc[d];
               const float sv = (rss[k] - rsc[d]) + av;
               const float s = sv - 0.5f * (av + r[k]);
-              ax = fmaf(mi[k] * av, s, ax);
-              ay = fmaf(mi[k] * r[k], s, ay);
+              if (DM) {
+                left[k] = av;
+                mid[k] = s;
+              } else {
+                ax = fmaf(mi[DM ? 0 : k] * av, s, ax);
+                ay = fmaf(mi[DM ? 0 : k] * r[k], s, ay);
+              }
             } else {
               rc[d] = r[k];
               rsc[d] = rss[k];
             }
           }
-          const FF v = warp_sum3ff(ff_from(kinf), ff_from(ax), ff_from(ay), lane);
-          if (idx == idx_max) kin = ff_from_lane(v, 0);
-          sub_turning = (__ballot_sync(FULL, ff_le0(v)) & ((1u << 8) | (1u << 16))) != 0u;
+          if (DM && odd) {
+            matvec(mid, v);
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+              ax = fmaf(left[k], v[k], ax);
+              ay = fmaf(r[k], v[k], ay);
+            }
+          }
+          const FF sums = warp_sum3ff(ff_from(kinf), ff_from(ax), ff_from(ay), lane);
+          if (idx == idx_max) kin = ff_from_lane(sums, 0);
+          sub_turning = (__ballot_sync(FULL, ff_le0(sums)) & ((1u << 8) | (1u << 16))) != 0u;
         }
         // ------------------------------------------------------ energy, divergence, multinomial choice
         const double e_new = pe + ff_value_int(FF{0.5f * kin.hi, 0.5f * kin.lo});
@@ -324,23 +402,39 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
       const float x = (float)dw;
       if (!(sub_turning || sub_div)) p = fminf(expf(x), 1.0f);
       float ax = 0.0f, ay = 0.0f;
+      float lr[K], rr[K], mid[K], v[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         const int d = lane + 32 * k;
+        if (DM) lr[k] = rr[k] = mid[k] = 0.0f;
         if (d < D) {
           const float sv = P.e.rsum[row + d] + rss[k];
           P.e.rsum[row + d] = sv;
           const float ro = P.e.r_l[row + d];
           const float av = dir ? ro : r[k], bv = dir ? r[k] : ro;  // left, right
           const float s = sv - 0.5f * (av + bv);
-          ax = fmaf(mi[k] * av, s, ax);
-          ay = fmaf(mi[k] * bv, s, ay);
+          if (DM) {
+            lr[k] = av;
+            rr[k] = bv;
+            mid[k] = s;
+          } else {
+            ax = fmaf(mi[DM ? 0 : k] * av, s, ax);
+            ay = fmaf(mi[DM ? 0 : k] * bv, s, ay);
+          }
+        }
+      }
+      if (DM) {
+        matvec(mid, v);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          ax = fmaf(lr[k], v[k], ax);
+          ay = fmaf(rr[k], v[k], ay);
         }
       }
       tree_turning = sub_turning;
       if (!tree_turning) {
-        const FF v = warp_sum3ff(ff_from(ax), ff_from(ay), FF{1.0f, 0.0f}, lane);
-        tree_turning = (__ballot_sync(FULL, ff_le0(v)) & ((1u << 0) | (1u << 8))) != 0u;
+        const FF sums = warp_sum3ff(ff_from(ax), ff_from(ay), FF{1.0f, 0.0f}, lane);
+        tree_turning = (__ballot_sync(FULL, ff_le0(sums)) & ((1u << 0) | (1u << 8))) != 0u;
       }
       if (u_take < p) {
         prop = sprop;
@@ -359,7 +453,7 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
       if (lane + 32 * k < D) P.e.Q[row + lane + 32 * k] = z[k];  // the last queried position
     const float* znew = prop < 0 ? P.s.z + row : (prop ? P.e.z_sp : P.e.z_p) + row;
     const float* gnew = prop < 0 ? P.s.z_grad + row : (prop ? P.e.g_sp : P.e.g_p) + row;
-    iters_left = hier_end_transition(P, hv, c, m, D, lane, pe_p, energy_p, num_prop, tree_acc / (double)num_prop,
+    iters_left = hier_end_transition<DM>(P, hv, c, m, D, lane, pe_p, energy_p, num_prop, tree_acc / (double)num_prop,
                                      tree_div, znew, gnew);
   }
 }
@@ -368,7 +462,7 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
 // models of 4 to 256 groups, 16,384 chains, 5 transitions), 20 took 4.4.  One K per launch: letting
 // each chain run the smallest instance that holds it was no faster (several loops share the
 // instruction caches then).
-template <int K>
+template <int K, bool DM>
 __global__ void __launch_bounds__(128, 3)
     persistent_hier_reg_kernel(const AdvParams* __restrict__ Pp, const __grid_constant__ HierView hv,
                                int32_t* queue_head, const int32_t* __restrict__ order, int ck_floats) {
@@ -376,7 +470,9 @@ __global__ void __launch_bounds__(128, 3)
   extern __shared__ float ck_smem[];
   const AdvParams& P = stage_params(Pp, &sp);
   const int lane = threadIdx.x & 31;
-  float* const ck_warp = ck_smem + (size_t)(threadIdx.x >> 5) * ck_floats;
+  const int mass_floats = DM ? P.D * (32 * K) : 0;
+  float* const minv = ck_smem + (size_t)(threadIdx.x >> 5) * (ck_floats + mass_floats);
+  float* const ck_warp = minv + mass_floats;
   for (;;) {
     int q = 0;
     if (lane == 0) q = atomicAdd(queue_head, 1);
@@ -386,7 +482,7 @@ __global__ void __launch_bounds__(128, 3)
     int m = c / hv.cpm;
     if (m >= hv.num_models) m = hv.num_models - 1;
     const int D = P.e.chain_dim ? P.e.chain_dim[c] : P.D;
-    hier_run_chain<K>(P, hv, c, m, D, lane, ck_warp, ck_floats);
+    hier_run_chain<K, DM>(P, hv, c, m, D, lane, ck_warp, ck_floats, minv);
   }
 }
 

@@ -1243,26 +1243,26 @@ __global__ void __launch_bounds__(256) persistent_sv_kernel(const AdvParams* __r
 // Shared memory of an SM for its chains' U-turn checkpoints (64, 96 and 180 KB: no faster).
 constexpr size_t HIER_CK_SMEM = 128 * 1024;
 
-template <int K>
+template <int K, bool DM>
 static void launch_hier_reg(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order, int C,
-                            int maxd, int sms, int optin, cudaStream_t st) {
+                            int D, int maxd, int sms, int optin, cudaStream_t st) {
   // few chains: a warp per SM before any SM takes two
-  const int warps = C <= sms ? 1 : (C <= 2 * sms ? 2 : 4);
-  const int resident = 12 / warps;  // CTAs per SM that the checkpoints' shared memory leaves room for
-  const size_t slot = sizeof(float) * 64 * K * warps;
+  const int warps = C <= sms ? 1 : (C <= 2 * sms || DM ? 2 : 4);
+  const int resident = 12 / warps;  // CTAs per SM that the shared memory leaves room for
+  const size_t slot = sizeof(float) * 64 * K * warps, mass = DM ? sizeof(float) * 32 * K * (size_t)D * warps : 0;
   const int need = (C + warps - 1) / warps;
   const int per_sm_needed = std::min(resident, (need + sms - 1) / sms);
-  const size_t budget = std::min((size_t)(HIER_CK_SMEM / per_sm_needed), (size_t)optin - 2048);
+  const size_t budget = std::min((size_t)(HIER_CK_SMEM / per_sm_needed), (size_t)optin - 2048 - mass);
   const int slots = (int)std::min((size_t)maxd, budget / slot);
-  const size_t smem = slot * slots;
-  cudaFuncSetAttribute(persistent_hier_reg_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = slot * slots + mass;
+  cudaFuncSetAttribute(persistent_hier_reg_kernel<K, DM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int blocks = need;
   if (need > sms) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_reg_kernel<K>, 32 * warps, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_reg_kernel<K, DM>, 32 * warps, smem);
     blocks = std::min(need, sms * std::max(per_sm, 1));
   }
-  persistent_hier_reg_kernel<K><<<blocks, 32 * warps, smem, st>>>(dP, hv, queue_head, order, slots * 64 * K);
+  persistent_hier_reg_kernel<K, DM><<<blocks, 32 * warps, smem, st>>>(dP, hv, queue_head, order, slots * 64 * K);
 }
 
 void launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order,
@@ -1271,23 +1271,33 @@ void launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* qu
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  // The register engine holds up to 288 dimensions (nine elements a lane); HMC, dense mass matrices and
-  // larger models run the state machine over memory.
-  if (nuts && !dense && D <= 288) {
-    if (D <= 32)
-      launch_hier_reg<1>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
-    else if (D <= 64)
-      launch_hier_reg<2>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
-    else if (D <= 96)
-      launch_hier_reg<3>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
-    else if (D <= 160)
-      launch_hier_reg<5>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
-    else if (D <= 224)
-      launch_hier_reg<7>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
-    else
-      launch_hier_reg<9>(dP, hv, queue_head, order, C, maxd, sms, optin, st);
+  // The register engine holds up to 288 dimensions (nine elements a lane), 96 with a dense mass matrix (in
+  // shared memory, up to 36 KB a chain); HMC and larger models run the state machine over memory.
+#define HIER_REG(K, DM) launch_hier_reg<K, DM>(dP, hv, queue_head, order, C, D, maxd, sms, optin, st)
+  if (nuts && D <= (dense ? 96 : 288)) {
+    if (dense) {
+      if (D <= 32)
+        HIER_REG(1, true);
+      else if (D <= 64)
+        HIER_REG(2, true);
+      else
+        HIER_REG(3, true);
+    } else if (D <= 32) {
+      HIER_REG(1, false);
+    } else if (D <= 64) {
+      HIER_REG(2, false);
+    } else if (D <= 96) {
+      HIER_REG(3, false);
+    } else if (D <= 160) {
+      HIER_REG(5, false);
+    } else if (D <= 224) {
+      HIER_REG(7, false);
+    } else {
+      HIER_REG(9, false);
+    }
     return;
   }
+#undef HIER_REG
   if (dense)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_kernel<true>, 256, 0);
   else

@@ -49,3 +49,14 @@ def test_register_engine_warmup_is_the_tick_engine(sizes):
     a, b = _run(model, "fused", **args), _run(model, "ticks", **args)
     for f in a:
         np.testing.assert_array_equal(a[f], b[f], err_msg=f)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("J,chains", [(1, 3), (8, 5), (30, 5), (31, 200), (62, 4), (63, 4), (94, 310), (95, 3)])
+def test_register_engine_dense_mass_is_the_tick_engine(J, chains):
+    """Dense mass matrices through a window end (their factors change), one to three elements a lane."""
+    args = dict(chains=chains, warmup=24, draws=3, dense_mass=True, max_tree_depth=6)
+    a, b = _run(_model([J]), "fused", **args), _run(_model([J]), "ticks", **args)
+    assert a["draw_num_steps"].max() > 3
+    for f in a:
+        np.testing.assert_array_equal(a[f], b[f], err_msg=f)
