@@ -82,103 +82,118 @@ void logreg_prior_consts(double prior_scale, int p, float* inv_var_f, double* pe
 //   residuals  R[row][c]  = y[row] - sum_p Xt[p][row] Bt[p][c]       (Xt = X^T, Bt = beta^T)
 //   adjoint    GB[c][p]   = sum_row R[row][c] X[row][p]              (split over row ranges)
 // X^T and a padded X are built once per model; beta^T is packed from the chains' positions each
-// tick.  64 x 64 tiles, 16-deep K steps double-buffered through registers; 4 x 4 outputs per
-// thread.  Residual sums of squares per (row tile, chain) leave the GEMM in FP64.
-constexpr int HS_BN = 64, HS_BK = 16;
+// tick.  Residual sums of squares per (row tile, chain) leave the GEMM in FP64 (BM / 16 rows each in FP32).
+//
+// Tiles of BM x 64 outputs, 4 x 8 a thread.  At 2000 x 1000 x 256 chains a GEMM has 512,000 outputs, under one
+// warp of 32 outputs a thread for each scheduler.  Bound: shared-memory reads (a 16-byte read of a warp takes
+// four cycles, broadcast or not, so 4 x 4 outputs a thread read 8 cycles for 4 of multiply-adds, 4 x 8 12
+// for 8).  cp.async runs HS_STAGES - 1 K steps ahead.
+constexpr int HS_BN = 64, HS_BK = 32, HS_STAGES = 2;
+constexpr int HS_SPLIT_ROWS = 16;  // a row range of the adjoint GEMM is a multiple of this
 constexpr int HS_MIN_BM = 32;     // smallest tile height offered to the tuner
 constexpr int HS_MAX_SPLITS = 8;  // most row ranges offered to the tuner for the adjoint GEMM
 
-// TM rows per thread: tiles of (16 TM) x 64 outputs, 256 threads.
-template <int TM>
-__global__ void __launch_bounds__(256) hs_sgemm_nn_kernel(const float* __restrict__ A, int lda,
-                                                          const float* __restrict__ B, int ldb, int M, int N,
-                                                          int K, int k_per_split, float* __restrict__ Out, int ldo,
-                                                          int64_t split_stride, const float* __restrict__ yv,
-                                                          double* __restrict__ part_rr, int ld_rr,
-                                                          const int32_t* pending) {
+template <int BM>
+__global__ void __launch_bounds__(BM * HS_BN / 32)
+    hs_sgemm_nn_kernel(const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, int M, int N, int K,
+                       int k_per_split, float* __restrict__ Out, int ldo, int64_t split_stride,
+                       const float* __restrict__ yv, double* __restrict__ part_rr, int ld_rr, const int32_t* pending) {
   if (pending && *pending == 0) return;
-  constexpr int BM = 16 * TM;
-  constexpr int AQ = BM / 4;  // float4 per K row of the A tile
-  __shared__ __align__(16) float As[2][HS_BK][BM];
-  __shared__ __align__(16) float Bs[2][HS_BK][HS_BN];
-  __shared__ float rr[16][HS_BN];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  constexpr int NTH = BM * HS_BN / 32, TX = HS_BN / 8, TY = BM / 4;
+  __shared__ __align__(16) float As[HS_STAGES][HS_BK][BM];
+  __shared__ __align__(16) float Bs[HS_STAGES][HS_BK][HS_BN];
+  constexpr int SQ_ROWS = BM / 16;  // rows a sum of squares takes in FP32
+  __shared__ float rr[TY * 4 / SQ_ROWS][HS_BN];
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * HS_BN;
   const int kb = blockIdx.z * k_per_split, ke = min(K, kb + k_per_split);
-  // per K step a thread stages one float4 of B (row lk, columns lc..lc+3) and, when tid < 4 BM,
-  // one float4 of A (row ak, columns ac..ac+3)
-  const int lk = tid >> 4, lc = (tid & 15) * 4;
-  const bool a_loader = tid < HS_BK * AQ;
-  const int ak = tid / AQ, ac = (tid % AQ) * 4;
-  auto load = [&](int k0, float4& av, float4& bv) {
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    av = (a_loader && k0 + ak < ke && m0 + ac < M)
-             ? *reinterpret_cast<const float4*>(A + (size_t)(k0 + ak) * lda + m0 + ac)
-             : zero;
-    bv = (k0 + lk < ke && n0 + lc < N) ? *reinterpret_cast<const float4*>(B + (size_t)(k0 + lk) * ldb + n0 + lc)
-                                       : zero;
+  const int steps = ke > kb ? (ke - kb + HS_BK - 1) / HS_BK : 0;
+  auto stage = [&](int step) {  // one K step of both operands; past the end an empty group
+    if (step < steps) {
+      const int k0 = kb + step * HS_BK, s = step % HS_STAGES;
+#pragma unroll
+      for (int q = tid; q < HS_BK * BM / 4; q += NTH) {
+        const int k = q / (BM / 4), m = 4 * (q % (BM / 4));
+        const bool in = k0 + k < ke && m0 + m < M;
+        cp_async16(&As[s][k][m], in ? A + (size_t)(k0 + k) * lda + m0 + m : A, in);
+      }
+#pragma unroll
+      for (int q = tid; q < HS_BK * HS_BN / 4; q += NTH) {
+        const int k = q / (HS_BN / 4), n = 4 * (q % (HS_BN / 4));
+        const bool in = k0 + k < ke && n0 + n < N;
+        cp_async16(&Bs[s][k][n], in ? B + (size_t)(k0 + k) * ldb + n0 + n : B, in);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float acc[TM][4] = {};
-  float4 av, bv;
-  load(kb, av, bv);
-  int buf = 0;
-  for (int k0 = kb; k0 < ke; k0 += HS_BK) {
-    if (a_loader) *reinterpret_cast<float4*>(&As[buf][ak][ac]) = av;
-    *reinterpret_cast<float4*>(&Bs[buf][lk][lc]) = bv;
-    __syncthreads();
-    if (k0 + HS_BK < ke) load(k0 + HS_BK, av, bv);  // next step's loads overlap this step's FMAs
+#pragma unroll
+  for (int i = 0; i < HS_STAGES - 1; ++i) stage(i);
+  float acc[4][8] = {};
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(HS_STAGES - 2) : "memory");
+    __syncthreads();  // this step has landed, and every thread is done with the stage filled next
+    stage(step + HS_STAGES - 1);
+    const int s = step % HS_STAGES;
 #pragma unroll
     for (int kk = 0; kk < HS_BK; ++kk) {
-      float aa[TM];
+      const float4 a4 = *reinterpret_cast<const float4*>(&As[s][kk][4 * ty]);
+      const float4 b4 = *reinterpret_cast<const float4*>(&Bs[s][kk][4 * tx]);
+      const float4 c4 = *reinterpret_cast<const float4*>(&Bs[s][kk][HS_BN / 2 + 4 * tx]);
+      const float aa[4] = {a4.x, a4.y, a4.z, a4.w}, bb[8] = {b4.x, b4.y, b4.z, b4.w, c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
-      for (int i = 0; i < TM; i += 2) {
-        const float2 a2 = *reinterpret_cast<const float2*>(&As[buf][kk][ty * TM + i]);
-        aa[i] = a2.x;
-        aa[i + 1] = a2.y;
-      }
-      const float4 b4 = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 4]);
-      const float bb[4] = {b4.x, b4.y, b4.z, b4.w};
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
     }
-    buf ^= 1;  // the other buffer was last read before this step's barrier
   }
   float* out = Out + (size_t)blockIdx.z * split_stride;
   if (yv == nullptr) {
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int m = m0 + ty * TM + i;
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + ty * 4 + i;
       if (m >= M) continue;
-      if (n0 + tx * 4 < N)
-        *reinterpret_cast<float4*>(out + (size_t)m * ldo + n0 + tx * 4) =
-            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int nn = n0 + h * (HS_BN / 2) + 4 * tx;
+        if (nn < N)
+          *reinterpret_cast<float4*>(out + (size_t)m * ldo + nn) =
+              make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
+      }
     }
     return;
   }
   // residual epilogue: R = y - acc, and per-chain sums of R^2 over this row tile
-  float sq[4] = {0.f, 0.f, 0.f, 0.f};
+  float sq[8] = {};
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int m = m0 + ty * TM + i;
-    if (m >= M) continue;
-    const float y = yv[m];
-    float r[4];
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + ty * 4 + i;
+    const bool in = m < M;
+    const float y = in ? yv[m] : 0.0f;
+    float r[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      r[j] = y - acc[i][j];
+    for (int j = 0; j < 8; ++j) {
+      r[j] = in ? y - acc[i][j] : 0.0f;
       sq[j] = fmaf(r[j], r[j], sq[j]);
     }
-    if (n0 + tx * 4 < N) *reinterpret_cast<float4*>(out + (size_t)m * ldo + n0 + tx * 4) = make_float4(r[0], r[1], r[2], r[3]);
-  }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) rr[ty][tx * 4 + j] = sq[j];
+    for (int h = 0; h < 2; ++h) {
+      const int nn = n0 + h * (HS_BN / 2) + 4 * tx;
+      if (in && nn < N)
+        *reinterpret_cast<float4*>(out + (size_t)m * ldo + nn) = make_float4(r[4 * h], r[4 * h + 1], r[4 * h + 2], r[4 * h + 3]);
+    }
+    if ((i + 1) % SQ_ROWS == 0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        rr[(4 * ty + i) / SQ_ROWS][(j >> 2) * (HS_BN / 2) + 4 * tx + (j & 3)] = sq[j];
+        sq[j] = 0.0f;
+      }
+    }
+  }
   __syncthreads();
-  if (tid < HS_BN && n0 + tid < N) {
+  for (int n = tid; n < HS_BN && n0 + n < N; n += NTH) {
     double t = 0.0;
-    for (int k = 0; k < 16; ++k) t += (double)rr[k][tid];
-    part_rr[(size_t)blockIdx.y * ld_rr + n0 + tid] = t;
+    for (int k = 0; k < TY * 4 / SQ_ROWS; ++k) t += (double)rr[k][n];
+    part_rr[(size_t)blockIdx.y * ld_rr + n0 + n] = t;
   }
 }
 
@@ -375,16 +390,16 @@ cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, 
       // R[row][c] = y[row] - sum_p X[row][p] beta_c[p]
       dim3 g1((npts + HS_BN - 1) / HS_BN, mt, 1);
       if (tm == 2)
-        hs_sgemm_nn_kernel<2><<<g1, 256, 0, st>>>(m.hs_xt, pad4(M), m.hs_bt, cp, M, npts, P, P, m.resid, cp, 0,
-                                                  m.y, m.part_rr, cp, pending);
+        hs_sgemm_nn_kernel<32><<<g1, 64, 0, st>>>(m.hs_xt, pad4(M), m.hs_bt, cp, M, npts, P, P, m.resid, cp, 0, m.y,
+                                                  m.part_rr, cp, pending);
       else
-        hs_sgemm_nn_kernel<4><<<g1, 256, 0, st>>>(m.hs_xt, pad4(M), m.hs_bt, cp, M, npts, P, P, m.resid, cp, 0,
-                                                  m.y, m.part_rr, cp, pending);
+        hs_sgemm_nn_kernel<64><<<g1, 128, 0, st>>>(m.hs_xt, pad4(M), m.hs_bt, cp, M, npts, P, P, m.resid, cp, 0, m.y,
+                                                   m.part_rr, cp, pending);
       // GB[s][c][p] = sum_{row in split s} R[row][c] X[row][p]
-      const int kps = (((M + splits - 1) / splits) + HS_BK - 1) / HS_BK * HS_BK;
+      const int kps = (((M + splits - 1) / splits) + HS_SPLIT_ROWS - 1) / HS_SPLIT_ROWS * HS_SPLIT_ROWS;
       dim3 g2((P + HS_BN - 1) / HS_BN, (npts + 63) / 64, splits);
-      hs_sgemm_nn_kernel<4><<<g2, 256, 0, st>>>(m.resid, cp, m.hs_xp, pp, npts, P, M, kps, m.part_gb, pp,
-                                                (int64_t)npts * pp, nullptr, nullptr, 0, pending);
+      hs_sgemm_nn_kernel<64><<<g2, 128, 0, st>>>(m.resid, cp, m.hs_xp, pp, npts, P, M, kps, m.part_gb, pp,
+                                                 (int64_t)npts * pp, nullptr, nullptr, 0, pending);
       horseshoe_finish_kernel<<<npts, 256, 0, st>>>(Q, npts, ld, P, m.n, m.part_gb, splits, pp, m.part_rr, cp, mt,
                                                     nc, PE, G, pending);
       break;
@@ -484,12 +499,11 @@ cudaError_t autotune_potential(ModelDev& m, const float* Q, int npts, double* PE
         }
       }
     } else if (m.family == 3) {
-      for (int tm : {2, 4})
-        for (int sp : {2, 4, 8}) {
-          t.hs_tm = tm;
-          t.hs_splits = sp;
-          cand.push_back(t);
-        }
+      // By rule, not by timing: both shapes set the order of FP32 sums, and a choice made by a few
+      // launches' times made a model's results differ between processes.
+      t.hs_tm = npts >= 128 && (int64_t)m.n * m.p >= 1000000 ? 4 : 2;
+      t.hs_splits = m.n <= 64 ? 2 : (m.n <= 200 ? 4 : 8);
+      cand.push_back(t);
     }
     float best = 1e30f;
     TuneParams pick = m.tune;
