@@ -303,7 +303,7 @@ struct __align__(16) AdvParams {
   uint16_t* hsf_bs;  // [3][hsf_total] bfloat16 bits: point c, feature k at c * hsf_kp + k
   int64_t hsf_N;
   int64_t hsf_total;
-  int32_t hsf_P, hsf_kp, hsf_splits, hsf_ldg, hsf_ld_rr, hsf_mtiles, hsf_nc, hsf_pad;
+  int32_t hsf_P, hsf_splits, hsf_ldg, hsf_ld_rr, hsf_mtiles, hsf_nc;
 };
 
 // ---------------------------------------------------------------- groups

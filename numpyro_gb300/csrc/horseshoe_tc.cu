@@ -11,14 +11,20 @@
 // accumulator that the epilogue drains after every 64-wide K block and sums in FP32 registers
 // (round to nearest); the five correction products (2^-8 smaller) share one accumulator for the
 // whole K range.
-//   GEMM1  A = beta splits [3][Cp][Kp], B = X splits [3][Np][Kp]  -> R^T[chain][row] = y - D,
+//   GEMM1  A = beta splits [3][Kp/8][Cp][8], B = X splits [3][Np][Kp]  -> R^T[chain][row] = y - D,
 //          written back as bf16 splits (GEMM2's A operand) with per-(row tile, chain) sums of R^2
-//   GEMM2  A = R^T splits [3][Cp][Np], B = X^T splits [3][Pp][Np] -> partials of X^T R per
+//   GEMM2  A = R^T splits [3][Np/8][Cp][8], B = X^T splits [3][Pp][Np] -> partials of X^T R per
 //          row range (split-K), reduced by horseshoe_finish_kernel
 // X and X^T are split once per model; beta is split from the chains' positions every tick.
-// One CTA: warp 0 TMA producer (3-stage ring of 72 KB), warp 1 MMA issuer, warps 2..5 epilogue
-// (one TMEM lane quadrant each).  Every mbarrier wait is bounded; on a timeout the CTA records an
-// error, drains its copies and MMAs (bounded), frees TMEM and returns.
+// The A operand is read from TMEM, two buffers of [128 chains][64] x 3 terms.  With both operands in shared memory
+// the 24 MMAs of a K block took 1,270 cycles (53 each); with A in TMEM they take 890 (37 each; the tensor core's
+// own rate is 32), and copies, barriers and FP64 in the epilogue's loop that went beside them no longer wait on
+// the same shared memory.  4 to 6 stages of B and tiles of 32 rows for GEMM1 (which fill more SMs) measured the same or worse.
+// At 2000 x 1000 x 256 chains a warm launch of GEMM1 takes 15.1 us and of GEMM2 10.6 us (19.9 and 11.1 us before).
+// One CTA: warp 0 TMA producer of B, warp 1 MMA issuer, warps 2..5 epilogue (one TMEM lane quadrant each),
+// warps 6..13 bring A from global memory to TMEM, four for the even K blocks and four for the odd ones, so
+// that a group has two blocks' time for its loads.  Every mbarrier wait is bounded; on a timeout the CTA
+// records an error, drains its copies and MMAs (bounded), frees TMEM and returns.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -35,23 +41,28 @@ namespace hstc {
 using namespace tc;
 
 constexpr int TM = 128;  // MMA M: chains per tile (TMEM lanes)
-constexpr int TN = 64;   // MMA N: rows (GEMM1) or features (GEMM2) per tile
+constexpr int TN = 64;   // MMA N: rows of the data (GEMM1) or features (GEMM2) per tile
 constexpr int TK = 64;   // K per stage: one 128-byte swizzle row of bf16
 constexpr int NSPL = 3;  // bf16 terms per operand
-constexpr int STAGES = 3;
-constexpr int A_SPLIT = TM * TK * 2;                     // 16 KB
-constexpr int B_SPLIT = TN * TK * 2;                     // 8 KB
-constexpr int STAGE_BYTES = NSPL * (A_SPLIT + B_SPLIT);  // 72 KB
-constexpr int OFF_MISC = STAGES * STAGE_BYTES;
-constexpr int NUM_BARS = 2 * STAGES + 5;  // full, empty per stage; hh full/empty x 2; done
-constexpr int SMEM_BYTES = OFF_MISC + 256 + 1024;  // + alignment slack
-constexpr int NUM_THREADS = 32 * 6;
-constexpr uint32_t TMEM_COLS = 256;  // hh accumulators at columns 0 and 64, corrections at 128
-constexpr uint32_t CORR_COL = 128;
 constexpr int NPAIRS = 6;  // (A term, B term): hh, hm, mh, hl, lh, mm
+constexpr int NUM_THREADS = 32 * 14;
+constexpr int STAGES = 6;  // B stages: with 144 KB, one CTA fills an SM, as its TMEM does
+constexpr int B_SPLIT = TN * TK * 2;
+constexpr int STAGE_BYTES = NSPL * B_SPLIT;
+constexpr int OFF_MISC = STAGES * STAGE_BYTES;
+constexpr int NUM_BARS = 2 * STAGES + 9;  // full, empty per stage; hh full/empty x 2; A full/empty x 2; done
+constexpr int SMEM_BYTES = OFF_MISC + 384 + TN * 4 + 1024;  // + y of the tile + alignment slack
+constexpr uint32_t TMEM_COLS = 512;
+constexpr uint32_t A_TERM = TK / 2, A_BUF = NSPL * A_TERM;  // TMEM columns of one term, of one A buffer
+constexpr uint32_t A_COL = TMEM_COLS - 2 * A_BUF;
+constexpr uint32_t CORR_COL = 2 * TN;  // hh accumulators at columns 0 and TN, corrections after
+static_assert(CORR_COL + TN <= A_COL, "TMEM holds the accumulators and two A buffers");
+static_assert(NUM_BARS * 8 + 8 <= 384, "barriers, TMEM address and abort flag fit their slot");
 
 struct GemmArgs {
   int mode;              // 1: residuals (GEMM1), 2: adjoint partials (GEMM2)
+  const __nv_bfloat16* a;  // [3][K / 8][a_rows_split][8]
+  size_t a_term;           // elements of one term
   int a_rows_split;      // rows of one split in A's tensor (Cp)
   int b_rows_split;      // rows of one split in B's tensor
   int kblocks;           // K / TK
@@ -59,7 +70,7 @@ struct GemmArgs {
   int n_valid;           // valid columns (rows of the data for GEMM1, features for GEMM2)
   // mode 1
   const float* y;
-  __nv_bfloat16* rt;  // R^T splits [3][Cp][rt_ld]
+  __nv_bfloat16* rt;  // R^T splits [3][rt_ld / 8][Cp][8]
   int rt_ld;
   double* part_rr;  // [column tiles][ld_rr]
   int ld_rr;
@@ -90,9 +101,7 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16& h, __nv_bfloat16&
   l = __float2bfloat16_rn(r1 - __bfloat162float(m));
 }
 
-__global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid_constant__ CUtensorMap ta,
-                                                                    const __grid_constant__ CUtensorMap tb,
-                                                                    GemmArgs G) {
+__global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid_constant__ CUtensorMap tb, GemmArgs G) {
   if (G.pending && *G.pending == 0) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -107,7 +116,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
   auto empty = [&](int s) { return smem_u32(&bars[STAGES + s]); };
   auto hfull = [&](int b) { return smem_u32(&bars[2 * STAGES + b]); };
   auto hempty = [&](int b) { return smem_u32(&bars[2 * STAGES + 2 + b]); };
-  const uint32_t done = smem_u32(&bars[2 * STAGES + 4]);
+  auto afull = [&](int b) { return smem_u32(&bars[2 * STAGES + 4 + b]); };
+  auto aempty = [&](int b) { return smem_u32(&bars[2 * STAGES + 6 + b]); };
+  const uint32_t done = smem_u32(&bars[2 * STAGES + 8]);
+  float* ys = reinterpret_cast<float*>(smem + OFF_MISC + 384);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) {
@@ -117,11 +129,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
     for (int b = 0; b < 2; ++b) {
       bar_init(hfull(b), 1);
       bar_init(hempty(b), 4);  // the four epilogue warps
+      bar_init(afull(b), 4);   // the four warps that bring this buffer
+      bar_init(aempty(b), 1);
     }
     bar_init(done, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (G.mode == 1 && threadIdx.x < TN)
+    ys[threadIdx.x] = n0 + (int)threadIdx.x < G.n_valid ? G.y[n0 + threadIdx.x] : 0.0f;
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)),
                  "r"(TMEM_COLS)
@@ -132,21 +148,20 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_holder;
+  auto load_b = [&](int i) {
+    const int s = i % STAGES;
+    bar_expect_tx(full(s), STAGE_BYTES);
+    for (int sp = 0; sp < NSPL; ++sp)
+      tma_load_2d(smem_u32(smem + s * STAGE_BYTES + sp * B_SPLIT), &tb, (kb0 + i) * TK, sp * G.b_rows_split + n0, full(s));
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
       int issued = 0;
       for (int i = 0; i < nkb; ++i) {
-        const int s = i % STAGES;
-        if (i >= STAGES && !bar_wait(empty(s), ((i / STAGES) - 1) & 1, abort_flag, G.err)) break;
-        const int kx = (kb0 + i) * TK;
-        uint8_t* st = smem + s * STAGE_BYTES;
-        bar_expect_tx(full(s), STAGE_BYTES);
-        for (int sp = 0; sp < NSPL; ++sp) {
-          tma_load_2d(smem_u32(st + sp * A_SPLIT), &ta, kx, sp * G.a_rows_split + m0, full(s));
-          tma_load_2d(smem_u32(st + NSPL * A_SPLIT + sp * B_SPLIT), &tb, kx, sp * G.b_rows_split + n0, full(s));
-        }
+        if (i >= STAGES && !bar_wait(empty(i % STAGES), ((i / STAGES) - 1) & 1, abort_flag, G.err)) break;
+        load_b(i);
         issued = i + 1;
       }
       if (*abort_flag) {  // drain copies still in flight before the CTA can exit
@@ -168,29 +183,61 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
     const uint64_t d0 = sdesc(smem_u32(smem), 16, 1024);  // stage 0, offset 0
     for (int i = 0; i < nkb; ++i) {
       const int s = i % STAGES, hb = i & 1;
-      if (!bar_wait_warp(full(s), (i / STAGES) & 1, abort_flag, G.err)) break;
-      if (i >= 2 && !bar_wait_warp(hempty(hb), ((i >> 1) - 1) & 1, abort_flag, G.err)) break;
+      if (!bar_wait3_warp(full(s), (i / STAGES) & 1, true, afull(hb), (i >> 1) & 1, true, hempty(hb),
+                          ((i >> 1) - 1) & 1, i >= 2, abort_flag, G.err))
+        break;
       tc_fence_after();
       const uint64_t st = sdesc_at(d0, (uint32_t)(s * STAGE_BYTES));
+      const uint32_t at = tmem + A_COL + (uint32_t)hb * A_BUF;  // 8 columns per 16 of K
 #pragma unroll
       for (int kk = 0; kk < TK / 16; ++kk)  // hh of this block into its own accumulator
-        mma_bf16_warp(tmem + (uint32_t)(hb * TN), sdesc_at(st, kk * 32), sdesc_at(st, NSPL * A_SPLIT + kk * 32), ID,
-                      kk > 0 ? 1u : 0u);
+        mma_bf16_tmem_a_warp(tmem + (uint32_t)(hb * TN), at + kk * 8, sdesc_at(st, kk * 32), ID, kk > 0 ? 1u : 0u);
       mma_commit_warp(hfull(hb));
+      // Corrections share one accumulator over the whole K range.  (Terms of B side by side in one MMA of 2 TN
+      // columns took a third fewer MMAs and 1.5 us off a tick, but sum the corrections in another order, and
+      // a trajectory of 32 leapfrog steps then ends 1e-4 elsewhere.)
 #pragma unroll
-      for (int p = 1; p < NPAIRS; ++p) {  // corrections accumulate over the whole K range
+      for (int p = 1; p < NPAIRS; ++p) {
 #pragma unroll
         for (int kk = 0; kk < TK / 16; ++kk)
-          mma_bf16_warp(tmem + CORR_COL, sdesc_at(st, kPairA[p] * A_SPLIT + kk * 32),
-                        sdesc_at(st, NSPL * A_SPLIT + kPairB[p] * B_SPLIT + kk * 32), ID,
-                        (i > 0 || p > 1 || kk > 0) ? 1u : 0u);
+          mma_bf16_tmem_a_warp(tmem + CORR_COL, at + kPairA[p] * A_TERM + kk * 8,
+                               sdesc_at(st, kPairB[p] * B_SPLIT + kk * 32), ID, (i > 0 || p > 1 || kk > 0) ? 1u : 0u);
       }
       mma_commit_warp(empty(s));
+      mma_commit_warp(aempty(hb));
     }
     __syncwarp();
     mma_commit_warp(done);
     // every MMA issued by this warp has completed before TMEM can be released
     for (uint32_t k = 0; k < WAIT_LIMIT && !bar_try(done, 0); ++k) {
+    }
+  } else if (warp >= 6) {
+    // ------------------------------------------------------------ A operand to TMEM (warps 6..13)
+    const int q = warp & 3, group = (warp - 6) >> 2;
+    const uint32_t lrow = (uint32_t)(q * 32) << 16;
+    const size_t oct = (size_t)G.a_rows_split * 8;  // 8 of K for every chain
+    const __nv_bfloat16* const src = G.a + (size_t)kb0 * (TK / 8) * oct + (size_t)(m0 + q * 32 + lane) * 8;
+    for (int i = group; i < nkb; i += 2) {
+      uint32_t v[NSPL][2][16];
+#pragma unroll
+      for (int sp = 0; sp < NSPL; ++sp)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint4 u = *reinterpret_cast<const uint4*>(src + sp * G.a_term + (size_t)(i * (TK / 8) + j) * oct);
+          uint32_t* const o = v[sp][j >> 2] + 4 * (j & 3);
+          o[0] = u.x; o[1] = u.y; o[2] = u.z; o[3] = u.w;
+        }
+      if (i >= 2 && !bar_wait_warp(aempty(group), ((i >> 1) - 1) & 1, abort_flag, G.err)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int sp = 0; sp < NSPL; ++sp)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          tmem_st16(tmem + lrow + A_COL + (uint32_t)group * A_BUF + sp * A_TERM + 16 * h, v[sp][h]);
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) bar_arrive(afull(group));
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
@@ -221,7 +268,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
     if (ok) ok = bar_wait(done, 0, abort_flag, G.err);
     if (ok) {
       tc_fence_after();
-      double rr = 0.0;
+      float sums[TN / 16];
 #pragma unroll
       for (int j = 0; j < TN / 16; ++j) {
         float v[16];
@@ -241,24 +288,25 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
           float sq = 0.0f;
 #pragma unroll
           for (int e = 0; e < 16; e += 2) {
-            const float ra = (c0 + e < G.n_valid) ? G.y[c0 + e] - v[e] : 0.0f;
-            const float rb = (c0 + e + 1 < G.n_valid) ? G.y[c0 + e + 1] - v[e + 1] : 0.0f;
+            const float ra = (c0 + e < G.n_valid) ? ys[16 * j + e] - v[e] : 0.0f;
+            const float rb = (c0 + e + 1 < G.n_valid) ? ys[16 * j + e + 1] - v[e + 1] : 0.0f;
             sq = fmaf(ra, ra, sq);
             sq = fmaf(rb, rb, sq);
             split3_pair(ra, rb, hw[e >> 1], mw[e >> 1], lw[e >> 1]);
           }
-          rr += (double)sq;
-          const size_t o = (size_t)chain * G.rt_ld + c0;
-          const size_t sstride = (size_t)G.a_rows_split * G.rt_ld;  // Cp rows per split
+          sums[j] = sq;
+          const size_t oct = (size_t)G.a_rows_split * 8;  // GEMM2's A operand: 8 rows for every chain
+          const size_t o = (size_t)(c0 >> 3) * oct + (size_t)chain * 8;
+          const size_t sstride = (size_t)G.a_rows_split * G.rt_ld;
           uint4* dh = reinterpret_cast<uint4*>(G.rt + o);
           uint4* dm = reinterpret_cast<uint4*>(G.rt + sstride + o);
           uint4* dl = reinterpret_cast<uint4*>(G.rt + 2 * sstride + o);
           dh[0] = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-          dh[1] = make_uint4(hw[4], hw[5], hw[6], hw[7]);
           dm[0] = make_uint4(mw[0], mw[1], mw[2], mw[3]);
-          dm[1] = make_uint4(mw[4], mw[5], mw[6], mw[7]);
           dl[0] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-          dl[1] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
+          dh[G.a_rows_split] = make_uint4(hw[4], hw[5], hw[6], hw[7]);
+          dm[G.a_rows_split] = make_uint4(mw[4], mw[5], mw[6], mw[7]);
+          dl[G.a_rows_split] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
         } else if (chain < G.npts) {
           float* dst = G.part_gb + ((size_t)blockIdx.z * G.npts + chain) * G.ldg + c0;
 #pragma unroll
@@ -266,7 +314,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
             if (c0 + e < G.ldg) *reinterpret_cast<float4*>(dst + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
         }
       }
-      if (G.mode == 1 && chain < G.npts) G.part_rr[(size_t)blockIdx.x * G.ld_rr + chain] = rr;
+      if (G.mode == 1 && chain < G.npts) {
+        double rr = 0.0;
+#pragma unroll
+        for (int j = 0; j < TN / 16; ++j) rr += (double)sums[j];
+        G.part_rr[(size_t)blockIdx.x * G.ld_rr + chain] = rr;
+      }
     }
   }
   tc_fence_before();
@@ -295,13 +348,13 @@ __global__ void split_matrix_kernel(const float* __restrict__ x, int64_t n, int 
 }
 
 // beta [npts] rows (centred: z[0:P]; non-centred: exp(log tau + log lambda) * unscaled) -> splits
-// [3][Cp][Kp] bf16, zero padding
+// [3][Kp / 8][Cp][8] bf16 (a warp that brings 8 features of 32 chains reads 512 bytes in a row), zero padding
 __global__ void split_beta_kernel(const float* __restrict__ Q, int npts, int ld, int P, int noncentred, int cp,
                                   int kp, __nv_bfloat16* __restrict__ out, const int32_t* pending) {
   if (pending && *pending == 0) return;
   const int64_t total = (int64_t)cp * kp;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i / kp), k = (int)(i % kp);
+    const int c = (int)((i >> 3) % cp), k = (int)((i >> 3) / cp) * 8 + (int)(i & 7);
     float v = 0.0f;
     if (c < npts && k < P) {
       const float* z = Q + (size_t)c * ld;
@@ -321,7 +374,7 @@ struct HsState {
   float* part_gb = nullptr;
   double* part_rr = nullptr;
   int* err = nullptr;
-  CUtensorMap tm_x, tm_xt, tm_b, tm_rt;
+  CUtensorMap tm_x, tm_xt;
   bool ok = false;
 };
 
@@ -389,8 +442,7 @@ cudaError_t horseshoe_tc_prepare(ModelDev& m, int points) {
     split_matrix_kernel<<<1024, 256>>>(m.x, m.n, m.p, 1, s->pp, s->np, s->xts);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    bool ok = hs_encode(&s->tm_x, s->xs, s->kp, 3 * s->np, TN) && hs_encode(&s->tm_xt, s->xts, s->np, 3 * s->pp, TN) &&
-              hs_encode(&s->tm_b, s->bs, s->kp, 3 * s->cp, TM) && hs_encode(&s->tm_rt, s->rts, s->np, 3 * s->cp, TM);
+    bool ok = hs_encode(&s->tm_x, s->xs, s->kp, 3 * s->np, TN) && hs_encode(&s->tm_xt, s->xts, s->np, 3 * s->pp, TN);
     if (!ok) return cudaErrorInvalidValue;
     e = cudaFuncSetAttribute(hs_tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return e;
@@ -442,7 +494,6 @@ bool horseshoe_tc_fusion(ModelDev& m, int npts, AdvParams* P) {
   P->hsf_N = m.n;
   P->hsf_total = (int64_t)s->cp * s->kp;
   P->hsf_P = m.p;
-  P->hsf_kp = s->kp;
   P->hsf_splits = s->splits;
   P->hsf_ldg = s->pp;
   P->hsf_ld_rr = s->cp;
@@ -466,6 +517,8 @@ cudaError_t horseshoe_tc_launch(ModelDev& m, const float* Q, int npts, double* P
                                                                                  s->bs, pending);
   GemmArgs g1{};
   g1.mode = 1;
+  g1.a = s->bs;
+  g1.a_term = (size_t)s->cp * s->kp;
   g1.a_rows_split = s->cp;
   g1.b_rows_split = s->np;
   g1.kblocks = s->kp / TK;
@@ -479,9 +532,11 @@ cudaError_t horseshoe_tc_launch(ModelDev& m, const float* Q, int npts, double* P
   g1.npts = npts;
   g1.err = s->err;
   g1.pending = pending;
-  hs_tc_gemm_kernel<<<dim3(s->np / TN, cp / TM, 1), NUM_THREADS, SMEM_BYTES, st>>>(s->tm_b, s->tm_x, g1);
+  hs_tc_gemm_kernel<<<dim3(s->np / TN, cp / TM, 1), NUM_THREADS, SMEM_BYTES, st>>>(s->tm_x, g1);
   GemmArgs g2{};
   g2.mode = 2;
+  g2.a = s->rts;
+  g2.a_term = (size_t)s->cp * s->np;
   g2.a_rows_split = s->cp;
   g2.b_rows_split = s->pp;
   g2.kblocks = s->np / TK;
@@ -492,7 +547,7 @@ cudaError_t horseshoe_tc_launch(ModelDev& m, const float* Q, int npts, double* P
   g2.ldg = s->pp;
   g2.err = s->err;
   g2.pending = pending;
-  hs_tc_gemm_kernel<<<dim3(s->pp / TN, cp / TM, s->splits), NUM_THREADS, SMEM_BYTES, st>>>(s->tm_rt, s->tm_xt, g2);
+  hs_tc_gemm_kernel<<<dim3(s->pp / TN, cp / TM, s->splits), NUM_THREADS, SMEM_BYTES, st>>>(s->tm_xt, g2);
   if (!fused_tick)
     horseshoe_finish_launch(Q, npts, m.D, m.p, m.n, s->part_gb, s->splits, s->pp, s->part_rr, s->cp, s->np / TN, nc,
                             PE, G, pending, st);

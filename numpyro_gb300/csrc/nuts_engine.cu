@@ -1033,7 +1033,7 @@ __global__ void __launch_bounds__(256) advance_kernel(const AdvParams* __restric
       const float r1 = v - __bfloat162float(hi);
       const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
       const __nv_bfloat16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
-      const size_t i = (size_t)c * P.hsf_kp + k;
+      const size_t i = ((size_t)(k >> 3) * P.hsf_ld_rr + c) * 8 + (k & 7);
       P.hsf_bs[i] = __bfloat16_as_ushort(hi);
       P.hsf_bs[P.hsf_total + i] = __bfloat16_as_ushort(mid);
       P.hsf_bs[2 * P.hsf_total + i] = __bfloat16_as_ushort(lo);
