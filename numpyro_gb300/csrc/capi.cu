@@ -550,12 +550,13 @@ static cudaError_t upload_params(gbn_handle h, cudaStream_t st) {
 // issues the same launches with the same arguments; the kernels read their parameters from
 // device memory).
 constexpr int TICK_BATCH = 16;
-static cudaError_t launch_tick_batch(gbn_handle h, cudaStream_t st) {
+// dependent: each kernel may start while the one before it ends (launch_tick).
+static cudaError_t launch_tick_batch(gbn_handle h, cudaStream_t st, bool dependent) {
   for (int k = 0; k < TICK_BATCH; ++k) {
     const int parity = k & 1;
-    launch_advance(h->dP, h->C, h->D, h->cta_per_chain, h->hp.dense != 0, parity, st);
+    launch_advance(h->dP, h->C, h->D, h->cta_per_chain, h->hp.dense != 0, parity, st, dependent);
     cudaError_t e = launch_potential(h->m, h->e.Q, h->C, h->e.PE, h->e.G, h->counters + 2 * parity, st,
-                                     h->hp.lrf_part_g != nullptr || h->hp.hsf_part_gb != nullptr);
+                                     h->hp.lrf_part_g != nullptr || h->hp.hsf_part_gb != nullptr, dependent);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -567,7 +568,7 @@ static void capture_tick_graph(gbn_handle h) {
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    cudaError_t el = launch_tick_batch(h, h->cap_stream);
+    cudaError_t el = launch_tick_batch(h, h->cap_stream, true);
     e = cudaStreamEndCapture(h->cap_stream, &g);
     if (el != cudaSuccess) e = el;
   }
@@ -599,7 +600,7 @@ static int tick_loop(gbn_handle h, cudaStream_t st, int64_t max_ticks) {
     if (h->tick_graph) {
       e = cudaGraphLaunch(h->tick_graph, st);
     } else {
-      e = launch_tick_batch(h, st);
+      e = launch_tick_batch(h, st, true);
       if (e == cudaSuccess && h->use_graphs && ticks > 0) capture_tick_graph(h);
     }
     if (e != cudaSuccess) return cuda_fail(h, e, "tick launch");
@@ -790,7 +791,7 @@ static cudaError_t build_async_graph(gbn_handle h) {
     cudaGraph_t body = np.conditional.phGraph_out[0];
     e = cudaStreamBeginCaptureToGraph(h->cap_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      cudaError_t el = launch_tick_batch(h, h->cap_stream);
+      cudaError_t el = launch_tick_batch(h, h->cap_stream, false);
       const int* tc_err = h->m.tc ? logreg_tc_error_ptr(h->m) : (h->m.hs_tc ? horseshoe_tc_error_ptr(h->m) : nullptr);
       launch_tick_condition((unsigned long long)ch, h->counters, (TICK_BATCH - 1) & 1, h->async_iter, tc_err,
                             h->err_word, h->cap_stream);

@@ -52,34 +52,6 @@ __device__ __forceinline__ FF ff_from_lane(FF v, int src) {
   return FF{__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src)};
 }
 
-// FP64 without the FP64 pipe.  On GB300 a dependent FP64 add takes 64 cycles and a conversion 66,
-// and an SM starts one warp's FP64 instruction every 19 (16) cycles, so the conversions and
-// comparisons around a leaf's energies are done on the words of the double.
-// (double)x, exact for every x
-__device__ __forceinline__ double f2d(float x) {
-  const uint32_t e = __float_as_uint(x) & 0x7f800000u;
-  const float n = e == 0u ? x * 16777216.0f : x;  // subnormals scaled by 2^24
-  const uint32_t b = __float_as_uint(n), a = b & 0x7fffffffu;
-  uint32_t bias = 896u << 20;
-  if (e == 0u) bias = (896u - 24u) << 20;
-  if (e == 0x7f800000u) bias = (2u * 896u) << 20;  // infinities and NaN
-  if (a == 0u) bias = 0u;
-  return __hiloint2double((int)((b & 0x80000000u) | ((a >> 3) + bias)), (int)(b << 29));
-}
-__device__ __forceinline__ double ff_value_int(FF a) { return f2d(a.hi) + f2d(a.lo); }
-__device__ __forceinline__ bool d_isnan(double x) {  // quiet NaN (what arithmetic gives)
-  return (uint32_t)(__double2hiint(x) & 0x7fffffff) > 0x7ff00000u;
-}
-__device__ __forceinline__ bool d_gt_pos(double x, double limit) {  // x > limit, limit > 0, x not NaN
-  return __double_as_longlong(x) > __double_as_longlong(limit);
-}
-// log(e^a + e^b) from diff = b - a: logaddexp_mixed with the difference shared with the caller
-__device__ __forceinline__ double logaddexp_diff(double a, double b, double diff, float x) {
-  const double top = __double2hiint(diff) >= 0 ? b : a;
-  const double sum = top + f2d(log1pf(expf(-fabsf(x))));
-  return __double_as_longlong(top) == (long long)0xfff0000000000000ull ? top : sum;
-}
-
 // Out of line: one copy of the generator per kernel instead of K + 3.  With 16 warps of an SM at
 // different places of the tree, the size of the leaf loop's code is what the instruction cache sees.
 __device__ __noinline__ uint4 hier_draw(Seed s, uint32_t chain, uint32_t n, uint32_t purpose, int idx, int sub) {
@@ -369,7 +341,7 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
           sub_turning = (__ballot_sync(FULL, ff_le0(sums)) & ((1u << 8) | (1u << 16))) != 0u;
         }
         // ------------------------------------------------------ energy, divergence, multinomial choice
-        const double e_new = pe + ff_value_int(FF{0.5f * kin.hi, 0.5f * kin.lo});
+        const double e_new = pe + ff_half(kin);
         double dE = e_new - energy0;
         if (d_isnan(dE)) dE = INFINITY;
         const double w = -dE;

@@ -102,7 +102,6 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16& h, __nv_bfloat16&
 }
 
 __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid_constant__ CUtensorMap tb, GemmArgs G) {
-  if (G.pending && *G.pending == 0) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_MISC);
@@ -148,19 +147,36 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_holder;
+  // B is the model's data: its first stages are on their way before the previous kernel (the state
+  // machine, or GEMM1) has ended.  Everything else read here is that kernel's.
   auto load_b = [&](int i) {
     const int s = i % STAGES;
     bar_expect_tx(full(s), STAGE_BYTES);
     for (int sp = 0; sp < NSPL; ++sp)
       tma_load_2d(smem_u32(smem + s * STAGE_BYTES + sp * B_SPLIT), &tb, (kb0 + i) * TK, sp * G.b_rows_split + n0, full(s));
   };
+  const int ahead = min(nkb, STAGES);
+  if (warp == 0 && lane == 0)
+    for (int i = 0; i < ahead; ++i) load_b(i);
+  tick_wait();
+  tick_trigger();
+  if (G.pending && *G.pending == 0) {  // no chain needs this potential: the copies land, TMEM goes back
+    if (warp == 0 && lane == 0)
+      for (int i = 0; i < ahead; ++i)
+        for (uint32_t k = 0; k < WAIT_LIMIT && !bar_try(full(i), 0); ++k) {
+        }
+    __syncthreads();
+    if (warp == 1)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    return;
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      int issued = 0;
-      for (int i = 0; i < nkb; ++i) {
-        if (i >= STAGES && !bar_wait(empty(i % STAGES), ((i / STAGES) - 1) & 1, abort_flag, G.err)) break;
+      int issued = ahead;
+      for (int i = STAGES; i < nkb; ++i) {
+        if (!bar_wait(empty(i % STAGES), ((i / STAGES) - 1) & 1, abort_flag, G.err)) break;
         load_b(i);
         issued = i + 1;
       }
@@ -503,7 +519,7 @@ bool horseshoe_tc_fusion(ModelDev& m, int npts, AdvParams* P) {
 }
 
 cudaError_t horseshoe_tc_launch(ModelDev& m, const float* Q, int npts, double* PE, float* G, const int32_t* pending,
-                                cudaStream_t st, bool fused_tick) {
+                                cudaStream_t st, bool fused_tick, bool dependent) {
   using namespace hstc;
   HsState* s = reinterpret_cast<HsState*>(m.hs_tc);
   if (!s || !s->ok) return cudaErrorNotSupported;
@@ -532,7 +548,8 @@ cudaError_t horseshoe_tc_launch(ModelDev& m, const float* Q, int npts, double* P
   g1.npts = npts;
   g1.err = s->err;
   g1.pending = pending;
-  hs_tc_gemm_kernel<<<dim3(s->np / TN, cp / TM, 1), NUM_THREADS, SMEM_BYTES, st>>>(s->tm_x, g1);
+  e = launch_tick(hs_tc_gemm_kernel, dim3(s->np / TN, cp / TM, 1), NUM_THREADS, SMEM_BYTES, st, dependent, s->tm_x, g1);
+  if (e != cudaSuccess) return e;
   GemmArgs g2{};
   g2.mode = 2;
   g2.a = s->rts;
@@ -547,7 +564,9 @@ cudaError_t horseshoe_tc_launch(ModelDev& m, const float* Q, int npts, double* P
   g2.ldg = s->pp;
   g2.err = s->err;
   g2.pending = pending;
-  hs_tc_gemm_kernel<<<dim3(s->pp / TN, cp / TM, s->splits), NUM_THREADS, SMEM_BYTES, st>>>(s->tm_xt, g2);
+  e = launch_tick(hs_tc_gemm_kernel, dim3(s->pp / TN, cp / TM, s->splits), NUM_THREADS, SMEM_BYTES, st, dependent,
+                  s->tm_xt, g2);
+  if (e != cudaSuccess) return e;
   if (!fused_tick)
     horseshoe_finish_launch(Q, npts, m.D, m.p, m.n, s->part_gb, s->splits, s->pp, s->part_rr, s->cp, s->np / TN, nc,
                             PE, G, pending, st);

@@ -72,11 +72,34 @@ struct SvView {
   double s_rate, nu_rate;
 };
 
+// Launches a kernel of the tick loop; dependent: it may start while its predecessor in the stream ends
+// (programmatic dependent launch, also when captured into a graph), for kernels that call tick_wait.
+template <typename... P, typename... A>
+cudaError_t launch_tick(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool dependent,
+                        A... args) {
+  if (!dependent) {  // a plain launch costs the host a microsecond less
+    kernel<<<grid, block, smem, st>>>(static_cast<P>(args)...);
+    return cudaGetLastError();
+  }
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 inline int pad4(int v) { return (v + 3) & ~3; }
 
 // nuts_engine.cu
 // a CTA per chain when cta_per_chain or D > 1024, else a warp per chain
-void launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity, cudaStream_t st);
+void launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity, cudaStream_t st,
+                    bool dependent);
 void launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order,
                             int C, int D, int maxd, bool nuts, bool dense, cudaStream_t st);
 // searches: a warmup window's end may start a step-size search in this run
@@ -106,9 +129,9 @@ cudaError_t ensure_potential_scratch(ModelDev& m, int points);
 void free_potential_scratch(ModelDev& m);
 // fused_tick: the tick engine's call, whose advance kernel fuses the tensor-core logistic and
 // horseshoe potentials' coefficient split and finish (logreg_tc_fusion, horseshoe_tc_fusion);
-// other potentials ignore it
+// other potentials ignore it.  dependent: as launch_tick, for the potentials whose kernels take it
 cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, float* G,
-                             const int32_t* pending, cudaStream_t st, bool fused_tick = false);
+                             const int32_t* pending, cudaStream_t st, bool fused_tick = false, bool dependent = false);
 // Times the candidate launch shapes of this model's potential at npts points (Q: any valid
 // [npts][D] positions; PE/G outputs) and stores the fastest in m.tune.  Decisions are cached per
 // process for each (device, family, shape, points), so every handle of a shape runs the same
@@ -125,8 +148,7 @@ void horseshoe_tc_free(ModelDev& m);
 int horseshoe_tc_error(const ModelDev& m);  // nonzero: a device wait timed out
 int* horseshoe_tc_error_ptr(const ModelDev& m);  // device address of that error word (or null)
 cudaError_t horseshoe_tc_launch(ModelDev& m, const float* Q, int npts, double* PE, float* G, const int32_t* pending,
-                                cudaStream_t st,
-                                bool fused_tick = false);
+                                cudaStream_t st, bool fused_tick = false, bool dependent = false);
 
 // logreg_tc.cu (tensor-core BF16 split-precision logistic potential)
 bool logreg_tc_supported(const ModelDev& m);

@@ -68,7 +68,6 @@ struct LogregTile {
 
 template <int CT, int NTH, int RG, int CG, int FG, int SP, int NB, int MINB>
 __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs A) {
-  if (A.pending && *A.pending == 0) return;
   using T = LogregTile<CT, NTH, RG, CG, FG, SP, NB>;
   constexpr int TX = T::TX, TY = T::TY, RT = T::RT;
   extern __shared__ __align__(16) float lr_smem[];
@@ -83,10 +82,6 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
   const int64_t ntiles = (A.n + RT - 1) / RT;
 
   for (int k = tid; k < NB * RT * SP; k += NTH) xs[k] = 0.0f;  // features past p stay zero
-  for (int k = tid; k < 4 * nc * CT; k += NTH) {
-    const int c = k / (4 * nc), d = k % (4 * nc);
-    bs[d * CT + c] = (d < p && c0 + c < A.npts) ? A.q[(size_t)(c0 + c) * A.ld + d] : 0.0f;
-  }
   __syncthreads();
   auto load_tile = [&](int64_t tile, int buf) {
     float* const dst = xs + buf * RT * SP;
@@ -134,6 +129,16 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
 
   int buf = 0;
   if (rg < ntiles) load_tile(rg, 0);
+  tick_wait();  // the data is on its way; the positions are the previous kernel's
+  tick_trigger();
+  if (A.pending && *A.pending == 0) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+  for (int k = tid; k < 4 * nc * CT; k += NTH) {
+    const int c = k / (4 * nc), d = k % (4 * nc);
+    bs[d * CT + c] = (d < p && c0 + c < A.npts) ? A.q[(size_t)(c0 + c) * A.ld + d] : 0.0f;
+  }
   for (int64_t tile = rg; tile < ntiles; tile += groups, buf ^= NB - 1) {
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();  // this tile has landed; every thread is done with the other buffer and with E
@@ -269,6 +274,8 @@ constexpr int LR_ORDERED = 128;
 __global__ void __launch_bounds__(256) logreg_fp32_finish_kernel(const LogregArgs A, int groups, float inv_var,
                                                                  double pe_const, double* __restrict__ pe,
                                                                  float* __restrict__ g) {
+  tick_wait();
+  tick_trigger();
   if (A.pending && *A.pending == 0) return;
   __shared__ float4 part[LR_ORDERED][16];
   const int c = blockIdx.x, tid = threadIdx.x, d4 = tid & 15, slice = tid >> 4;
@@ -341,7 +348,8 @@ inline int logreg_fp32_row_groups(int64_t n, int npts, int want) {
 }
 
 template <int CT, int NTH, int RG, int CG, int FG, int NB32, int NB64, int MINB>
-static cudaError_t logreg_fp32_launch_variant(const LogregArgs& A, int row_groups, bool attr, cudaStream_t st) {
+static cudaError_t logreg_fp32_launch_variant(const LogregArgs& A, int row_groups, bool attr, cudaStream_t st,
+                                              bool dependent) {
   const int dp = (A.p + 3) / 4 * 4;
   const dim3 grid((A.npts + CT - 1) / CT, row_groups);
   if (attr) {  // the shared-memory limit, at the most features each instance takes
@@ -355,25 +363,23 @@ static cudaError_t logreg_fp32_launch_variant(const LogregArgs& A, int row_group
     return e;
   }
   if (dp <= 32)
-    logreg_fp32_kernel<CT, NTH, RG, CG, FG, 32, NB32, MINB>
-        <<<grid, NTH, LogregTile<CT, NTH, RG, CG, FG, 32, NB32>::bytes(dp), st>>>(A);
-  else
-    logreg_fp32_kernel<CT, NTH, RG, CG, FG, 64, NB64, MINB>
-        <<<grid, NTH, LogregTile<CT, NTH, RG, CG, FG, 64, NB64>::bytes(dp), st>>>(A);
-  return cudaGetLastError();
+    return launch_tick(logreg_fp32_kernel<CT, NTH, RG, CG, FG, 32, NB32, MINB>, grid, NTH,
+                       LogregTile<CT, NTH, RG, CG, FG, 32, NB32>::bytes(dp), st, dependent, A);
+  return launch_tick(logreg_fp32_kernel<CT, NTH, RG, CG, FG, 64, NB64, MINB>, grid, NTH,
+                     LogregTile<CT, NTH, RG, CG, FG, 64, NB64>::bytes(dp), st, dependent, A);
 }
 
 // variant < 0: sets every variant's shared-memory limit on the current device
-static cudaError_t logreg_fp32_launch(int variant, const LogregArgs& A, int row_groups, cudaStream_t st) {
+static cudaError_t logreg_fp32_launch(int variant, const LogregArgs& A, int row_groups, cudaStream_t st, bool dependent) {
   const bool attr = variant < 0;
   cudaError_t e = cudaSuccess;
-  if (attr || variant == 0) e = logreg_fp32_launch_variant<8, 32, 1, 1, 1, 2, 2, 6>(A, row_groups, attr, st);
+  if (attr || variant == 0) e = logreg_fp32_launch_variant<8, 32, 1, 1, 1, 2, 2, 6>(A, row_groups, attr, st, dependent);
   if ((attr && e == cudaSuccess) || variant == 1)
-    e = logreg_fp32_launch_variant<16, 64, 1, 1, 1, 2, 2, 5>(A, row_groups, attr, st);
+    e = logreg_fp32_launch_variant<16, 64, 1, 1, 1, 2, 2, 5>(A, row_groups, attr, st, dependent);
   if ((attr && e == cudaSuccess) || variant == 2)
-    e = logreg_fp32_launch_variant<64, 256, 1, 1, 1, 2, 2, 2>(A, row_groups, attr, st);
+    e = logreg_fp32_launch_variant<64, 256, 1, 1, 1, 2, 2, 2>(A, row_groups, attr, st, dependent);
   if ((attr && e == cudaSuccess) || variant == 3)
-    e = logreg_fp32_launch_variant<128, 256, 1, 2, 1, 2, 2, 2>(A, row_groups, attr, st);
+    e = logreg_fp32_launch_variant<128, 256, 1, 2, 1, 2, 2, 2>(A, row_groups, attr, st, dependent);
   return e;
 }
 

@@ -165,7 +165,7 @@ struct Chain {
       for (int k = 0; k < UB; ++k)
         if (d0 + k * NT < D) acc = fmaf(mm[k] * rr[k], rr[k], acc);
     }
-    return 0.5 * ff_value(g.sumff(ff_from(acc), red));
+    return ff_half(g.sumff(ff_from(acc), red));
   }
 
   // _is_turning: v_l . (rs - (r_l + r_r)/2) <= 0 or v_r . (...) <= 0, with v = M^-1 r;
@@ -237,7 +237,7 @@ struct Chain {
     g.sync();
     float acc = 0.0f;
     sym_matvec(MX(P.s.inverse_mass_matrix), r, [&](int d, float v) { acc = fmaf(v, r[d], acc); });
-    return 0.5 * ff_value(g.sumff(ff_from(acc), red));
+    return ff_half(g.sumff(ff_from(acc), red));
   }
   // _is_turning with a dense M^-1: v_l . s = r_l . (M^-1 s) as M^-1 is symmetric
   __device__ bool is_turning_dense(const float* rl, const float* rr, const float* rs, const float* rs_minus,
@@ -345,7 +345,7 @@ struct Chain {
         acc = fmaf(mm[k] * rn, rn, acc);
       }
     }
-    return 0.5 * ff_value(g.sumff(ff_from(acc), red));
+    return ff_half(g.sumff(ff_from(acc), red));
   }
 
   __device__ float signed_step() const { return ctl.dir ? ctl.step : -ctl.step; }
@@ -400,7 +400,7 @@ struct Chain {
         rl[d] = r; rr[d] = r; rs[d] = r;
       }
     }
-    const double kin0 = DM ? kin_dense : 0.5 * ff_value(g.sumff(ff_from(kin), red));
+    const double kin0 = DM ? kin_dense : ff_half(g.sumff(ff_from(kin), red));
     int i = P.s.i[c];
     double pe = P.s.potential_energy[c];
     ctl.energy0 = pe + kin0;
@@ -450,10 +450,10 @@ struct Chain {
     double pe = P.e.PE[c];
     double e_new = pe + kin;
     double dE = e_new - ctl.energy0;
-    if (isnan(dE)) dE = INFINITY;
+    if (d_isnan(dE)) dE = INFINITY;
     double w = -dE;
-    int div = dE > P.max_dE;
-    double acc = (double)exp_min1_f(-dE);
+    int div = d_gt_pos(dE, P.max_dE);
+    double acc = f2d(exp_min1_f(w));
     const float* zf = (right ? z_r_() : z_l_());
     const float* rf = (right ? r_r_() : r_l_());
     const float* gf = (right ? g_r_() : g_l_());
@@ -486,7 +486,9 @@ struct Chain {
       ctl.energy_sp = e_new;
       ctl.sub_acc = acc;
     } else {
-      const float p = sigmoid_f(w - ctl.sub_w);
+      const double dw = w - ctl.sub_w;
+      const float x = (float)dw;
+      const float p = 1.0f / (1.0f + expf(-x));  // sigmoid_f(w - sub_w)
       uint4 u = draw(P.seed, chain_id, n, P_LEAF, (uint32_t)ctl.depth, (uint32_t)leaf_idx);
       bool take = u01f(u.x) < p;
       for (int d0 = g.tid; d0 < D; d0 += UB * NT) {
@@ -515,7 +517,7 @@ struct Chain {
         ctl.pe_sp = pe;
         ctl.energy_sp = e_new;
       }
-      ctl.sub_w = logaddexp_mixed(ctl.sub_w, w);
+      ctl.sub_w = logaddexp_diff(ctl.sub_w, w, dw, x);
       ctl.sub_acc += acc;
     }
     ctl.sub_div = div;
@@ -749,7 +751,7 @@ struct Chain {
       rh[d] = h;
       put_q(q, d, z[d] + eps * (mi[d] * h));
     }
-    ctl.heur_e0 = P.s.potential_energy[c] + 0.5 * ff_value(g.sumff(ff_from(kin), red));
+    ctl.heur_e0 = P.s.potential_energy[c] + ff_half(g.sumff(ff_from(kin), red));
     ctl.phase = PH_HEUR;
   }
   // returns true when the search is over (step size in ctl.heur_step)
@@ -769,7 +771,7 @@ struct Chain {
         float rn = rh[d] - 0.5f * eps * G[d];
         kin = fmaf(mi[d] * rn, rn, kin);
       }
-      e_new = P.e.PE[c] + 0.5 * ff_value(g.sumff(ff_from(kin), red));
+      e_new = P.e.PE[c] + ff_half(g.sumff(ff_from(kin), red));
     }
     double dE = e_new - ctl.heur_e0;
     int dir_new = (log(0.8) < -dE) ? 1 : -1;
@@ -900,9 +902,9 @@ struct Chain {
         double pe = P.e.PE[c];
         double e_new = pe + kin;
         double dE = e_new - ctl.energy0;
-        if (isnan(dE)) dE = INFINITY;
-        double acc = (double)exp_min1_f(-dE);
-        int div = dE > P.max_dE;
+        if (d_isnan(dE)) dE = INFINITY;
+        double acc = f2d(exp_min1_f(-dE));
+        int div = d_gt_pos(dE, P.max_dE);
         uint32_t n = P.s.rng_key[2 * c + 1];
         uint32_t chain_id = P.s.rng_key[2 * c];
         uint4 u = draw(P.seed, chain_id, n, P_HMC_ACCEPT, 0, 0);
@@ -989,6 +991,8 @@ __global__ void __launch_bounds__(256) advance_kernel(const AdvParams* __restric
     c = blockIdx.x;
     tid = threadIdx.x;
   }
+  tick_wait();  // the parameter block above is written before the tick loop
+  tick_trigger();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     P.counters[2 * (parity ^ 1)] = 0;
     P.counters[2 * (parity ^ 1) + 1] = 0;
@@ -1379,15 +1383,14 @@ void launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t* queue_
     persistent_sv_kernel<false><<<blocks, 256, 0, st>>>(dP, sv, queue_head);
 }
 
-void launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity, cudaStream_t st) {
+void launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity, cudaStream_t st,
+                    bool dependent) {
   if (!cta_per_chain && D <= 1024) {
-    int cpb = 8;
-    if (dense)
-      advance_kernel<32, true><<<(C + cpb - 1) / cpb, 32 * cpb, 0, st>>>(dP, parity);
-    else
-      advance_kernel<32, false><<<(C + cpb - 1) / cpb, 32 * cpb, 0, st>>>(dP, parity);
-  } else {
-    advance_kernel<256, false><<<C, 256, 0, st>>>(dP, parity);  // dense mass needs a warp per chain
+    const int cpb = 8;
+    launch_tick(dense ? advance_kernel<32, true> : advance_kernel<32, false>, (C + cpb - 1) / cpb, 32 * cpb, 0, st,
+                dependent, dP, parity);
+  } else {  // dense mass needs a warp per chain
+    launch_tick(advance_kernel<256, false>, C, 256, 0, st, dependent, dP, parity);
   }
 }
 

@@ -333,28 +333,28 @@ cudaError_t logreg_simt_smem_attr() {
   LogregArgs probe{};
   probe.p = 1;
   probe.npts = 1;
-  e = logreg_fp32_launch(-1, probe, 1, 0);
+  e = logreg_fp32_launch(-1, probe, 1, 0, false);
   if (e == cudaSuccess) g_simt_attr_done[(size_t)dev] = 1;
   return e;
 }
 
 static cudaError_t launch_logreg_fp32(const float* x, const float* y, int64_t n, int p, double prior_scale,
                                       const float* Q, int npts, int ld, int row_groups, float* part_g, double* part_ll,
-                                      double* PE, float* G, const int32_t* pending, cudaStream_t st) {
+                                      double* PE, float* G, const int32_t* pending, cudaStream_t st,
+                                      bool dependent) {
   cudaError_t e = logreg_simt_smem_attr();
   if (e != cudaSuccess) return e;
   const LogregArgs A{x, y, n, p, Q, npts, ld, part_g, part_ll, pending};
-  e = logreg_fp32_launch(logreg_fp32_shape(n, npts).variant, A, row_groups, st);
+  e = logreg_fp32_launch(logreg_fp32_shape(n, npts).variant, A, row_groups, st, dependent);
   if (e != cudaSuccess) return e;  // checked per launch, so the first failing launch is the one reported
   float ivf;
   double pec;
   logreg_prior_consts(prior_scale, p, &ivf, &pec);
-  logreg_fp32_finish_kernel<<<npts, 256, 0, st>>>(A, row_groups, ivf, pec, PE, G);
-  return cudaGetLastError();
+  return launch_tick(logreg_fp32_finish_kernel, npts, 256, 0, st, dependent, A, row_groups, ivf, pec, PE, G);
 }
 
 cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, float* G, const int32_t* pending,
-                             cudaStream_t st, bool fused_tick) {
+                             cudaStream_t st, bool fused_tick, bool dependent) {
   if (npts <= 0) return cudaSuccess;
   cudaError_t e = ensure_potential_scratch(m, npts);
   if (e != cudaSuccess) return e;
@@ -374,12 +374,13 @@ cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, 
       const int want = npts == m.scratch_points ? m.tune.lr_rg : 0;
       const int rg = (int)std::min<int64_t>(logreg_fp32_row_groups(m.n, npts, want),
                                             (int64_t)m.row_groups_cap * m.scratch_points / npts);
-      e = launch_logreg_fp32(m.x, m.y, m.n, m.p, m.hyper[0], Q, npts, ld, rg, m.part_g, m.part_ll, PE, G, pending, st);
+      e = launch_logreg_fp32(m.x, m.y, m.n, m.p, m.hyper[0], Q, npts, ld, rg, m.part_g, m.part_ll, PE, G, pending, st,
+                             dependent);
       if (e != cudaSuccess) return e;
       break;
     }
     case 3: {
-      if (m.precision == 1 && m.hs_tc) return horseshoe_tc_launch(m, Q, npts, PE, G, pending, st, fused_tick);
+      if (m.precision == 1 && m.hs_tc) return horseshoe_tc_launch(m, Q, npts, PE, G, pending, st, fused_tick, dependent && fused_tick);
       const int P = m.p, M = (int)m.n, cp = pad4(npts), pp = pad4(P);
       const int tm = m.tune.hs_tm, splits = m.tune.hs_splits, bm = 16 * tm;
       const int mt = (M + bm - 1) / bm;
@@ -613,7 +614,7 @@ cudaError_t launch_logreg_simt_scratch(const float* x, const float* y, int64_t n
                                        const float* Q, int npts, int row_groups, float* part_g, double* part_ll,
                                        double* PE, float* G, cudaStream_t st) {
   return launch_logreg_fp32(x, y, n, p, prior_scale, Q, npts, p, logreg_fp32_row_groups(n, npts, row_groups), part_g,
-                            part_ll, PE, G, nullptr, st);
+                            part_ll, PE, G, nullptr, st, false);
 }
 
 void horseshoe_finish_launch(const float* Q, int npts, int ld, int P, int64_t N, const float* part_gb, int splits,

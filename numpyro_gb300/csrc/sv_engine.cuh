@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(320, 2)
           for (int i = lane + 32; i <= 2 * checks; i += 32) turn = turn || ff_le0(sv_fold(sm.r2, i));
           sub_turning = __any_sync(FULL, turn);
           const FF kin = ff_from_lane(v, 0);
-          const double pe_leaf = sm.pe, e_new = pe_leaf + ff_value_int(FF{0.5f * kin.hi, 0.5f * kin.lo});
+          const double pe_leaf = sm.pe, e_new = pe_leaf + ff_half(kin);
           double dE = e_new - energy0;
           if (d_isnan(dE)) dE = INFINITY;
           const double w = -dE;
