@@ -245,20 +245,114 @@ __global__ void __launch_bounds__(256) horseshoe_finish_kernel(const float* __re
 }
 
 // ============================================================ stochastic volatility
-// z = [h(T) or h_base(T), log nu, log s]; CTA per point (sv_potential.cuh).
-__global__ void __launch_bounds__(256) sv_kernel(const float* __restrict__ Q, int npts, int ld, int T,
-                                                 const float* __restrict__ ret, double s_rate, double nu_rate,
-                                                 int noncentred, double* __restrict__ PE, float* __restrict__ G,
-                                                 const int32_t* pending) {
+// z = [h(T) or h_base(T), log nu, log s]; CTA per point (sv_potential.cuh): non-centred walks of more than
+// SV_REG_CHUNK steps a thread.
+__global__ void __launch_bounds__(256) sv_nc_long_kernel(const float* __restrict__ Q, int ld, int T,
+                                                         const float* __restrict__ ret, double s_rate, double nu_rate,
+                                                         double* __restrict__ PE, float* __restrict__ G,
+                                                         const int32_t* pending) {
   if (pending && *pending == 0) return;
   __shared__ SvSmem<256> sm;
-  const int c = blockIdx.x, tid = threadIdx.x;
-  const float* z = Q + (size_t)c * ld;
-  float* gz = G + (size_t)c * ld;
-  if (noncentred)
-    sv_nc_potential_block<256>(z, gz, PE + c, T, ret, s_rate, nu_rate, tid, sm);
-  else
-    sv_potential_block<256>(z, gz, PE + c, T, ret, s_rate, nu_rate, tid, sm);
+  const size_t c = blockIdx.x;
+  sv_nc_potential_block<256>(Q + c * ld, G + c * ld, PE + c, T, ret, s_rate, nu_rate, threadIdx.x, sm);
+}
+
+// CTA per point: eight element warps, and two scalar warps for what is FP64 or long (on GB300 a log-gamma takes
+// 1,700 to 3,100 cycles, a dependent FP64 operation 64): warp 8 the digammas, warp 9 the log-gammas, beside
+// the elements; then U in warp 9, dU/d log nu in warp 8 and dU/d log s in warp 0 beside one another.  With one
+// thread for all of it after the elements, and the log-gammas in front of two element warps, a point took
+// 20,000 cycles.  NC: the walk's rows pass through shared memory, as a thread's steps are consecutive.
+// Arithmetic and order of the sums are the block functions', so all engines give the same bits.
+// 4,096 steps x 1,024 points, non-centred: 53 -> 37 us (41 with two blocks an SM; 48 registers for four are no faster).  What is left
+// is issue: 218 instructions a step, most of them the seven compensated sums, at 2.7 a cycle and SM.
+template <int K, bool NC>
+__global__ void __launch_bounds__(320, 3) sv_potential_kernel(const float* __restrict__ Q, int ld, int T,
+                                                           const float* __restrict__ ret, double s_rate,
+                                                           double nu_rate, double* __restrict__ PE,
+                                                           float* __restrict__ G, const int32_t* pending) {
+  if (pending && *pending == 0) return;
+  __shared__ float2 r1[5][8], wt[2][8];
+  extern __shared__ float rows[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* const z = Q + (size_t)blockIdx.x * ld;
+  float* const g = G + (size_t)blockIdx.x * ld;
+  const float lnuf = z[T], lsf = z[T + 1];
+  float* const zs = rows;
+  float* const rets = rows + sv_pos(T) + 1;
+  if (NC && warp < 8) {
+    float a[K], b[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const bool in = tid + 256 * k < T;
+      a[k] = in ? z[tid + 256 * k] : 0.0f;
+      b[k] = in ? ret[tid + 256 * k] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (tid + 256 * k < T) {
+        zs[sv_pos(tid + 256 * k)] = a[k];
+        rets[sv_pos(tid + 256 * k)] = b[k];
+      }
+    asm volatile("bar.sync 2, 256;" ::: "memory");
+  }
+  const float nuf = expf(lnuf), sf = expf(lsf), inv_nuf = 1.0f / nuf;
+  float dg = 0.0f;
+  double lg = 0.0;
+  if (warp == 9) {
+    const double nu = (double)nuf;
+    lg = lgamma(0.5 * (lane == 1 ? nu + 1.0 : nu));
+  } else if (warp == 8) {
+    dg = digamma_f(0.5f * (lane == 1 ? nuf + 1.0f : nuf));
+  } else if (NC) {
+    sv_nc_elements<K>(zs, rets, rets, T, tid, sf, nuf, inv_nuf, r1, wt);
+  } else {
+    const float inv_s2 = 1.0f / (sf * sf);
+    Comp32 sdd{0.0f, 0.0f}, sl1p{0.0f, 0.0f}, sfrac{0.0f, 0.0f}, sh{0.0f, 0.0f};
+    for (int t0 = tid; t0 < T; t0 += K * 256) {  // loads of K steps are issued before their gradient stores
+      float hv[K], hp[K], hn[K], rv[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int t = t0 + k * 256;
+        hv[k] = t < T ? z[t] : 0.0f;
+        hp[k] = (t < T && t > 0) ? z[t - 1] : 0.0f;
+        hn[k] = (t + 1 < T) ? z[t + 1] : 0.0f;
+        rv[k] = t < T ? ret[t] : 0.0f;
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int t = t0 + k * 256;
+        if (t < T) g[t] = sv_centred_step(t, T, hv[k], hp[k], hn[k], rv[k], nuf, inv_nuf, inv_s2, sdd, sl1p, sfrac, sh);
+      }
+    }
+    const FF v = warp_sum4ff(comp_ff(sdd), comp_ff(sl1p), comp_ff(sfrac), comp_ff(sh), lane);
+    if ((lane & 7) == 0) r1[lane >> 3][warp] = make_float2(v.hi, v.lo);
+  }
+  __syncthreads();
+  if (NC && warp < 8)
+    for (int t = tid; t < T; t += 256) g[t] = rets[sv_pos(t)];
+  if (warp >= 8 || warp == 0) {
+    const double sums = ff_value(sv_fold(r1, lane < (NC ? 5 : 4) ? lane : 0));
+    const double nu = (double)nuf, s = (double)sf, inv_s = (double)(1.0f / sf);
+    const uint32_t FULL = 0xffffffffu;
+    const double S0 = __shfl_sync(FULL, sums, 0), S1 = __shfl_sync(FULL, sums, 1), S2 = __shfl_sync(FULL, sums, 2),
+                 S3 = __shfl_sync(FULL, sums, 3), S4 = __shfl_sync(FULL, sums, 4);
+    const double S_l1p = NC ? S0 : S1, S_frac = NC ? S1 : S2, S_h = NC ? S2 : S3;
+    if (warp == 8) {
+      const double special[6] = {0.0, 0.0, (double)__shfl_sync(FULL, dg, 0), (double)__shfl_sync(FULL, dg, 1), nu,
+                                 (double)inv_nuf};
+      const float gl = sv_grad_lnu(S_l1p, S_frac, (double)T, nu_rate, special);
+      if (lane == 0) g[T] = gl;
+    } else if (warp == 9) {
+      const double lg0 = __shfl_sync(FULL, lg, 0), lg1 = __shfl_sync(FULL, lg, 1);
+      const double log_rates = (double)(logf((float)s_rate) + logf((float)nu_rate));
+      const double pe = -sv_log_joint(NC, NC ? S4 : S0, S_l1p, S_h, (double)T, lnuf, lsf, nu, s, inv_s, log_rates, s_rate,
+                                      nu_rate, lg0, lg1);
+      if (lane == 0) PE[blockIdx.x] = pe;
+    } else {
+      const float gl = sv_grad_ls(NC, NC ? S3 : S0, (double)T, s, inv_s, s_rate);
+      if (lane == 0) g[T + 1] = gl;
+    }
+  }
 }
 
 __global__ void scale_rows_kernel(const double* __restrict__ cot, float* __restrict__ G, int npts, int D) {
@@ -353,6 +447,31 @@ static cudaError_t launch_logreg_fp32(const float* x, const float* y, int64_t n,
   return launch_tick(logreg_fp32_finish_kernel, npts, 256, 0, st, dependent, A, row_groups, ivf, pec, PE, G);
 }
 
+// Steps a thread: those of the walk, rounded up to the next instance.
+static void launch_sv(const float* Q, int npts, int ld, int T, const float* ret, double s_rate, double nu_rate,
+                      bool noncentred, double* PE, float* G, const int32_t* pending, cudaStream_t st) {
+  const int chunk = (T + 255) / 256;
+  const size_t smem = noncentred ? sizeof(float) * 2 * (size_t)(T + T / 16 + 1) : 0;
+#define SV_POTENTIAL(K, NC) \
+  sv_potential_kernel<K, NC><<<npts, 320, smem, st>>>(Q, ld, T, ret, s_rate, nu_rate, PE, G, pending)
+  if (noncentred && chunk > SV_REG_CHUNK)
+    sv_nc_long_kernel<<<npts, 256, 0, st>>>(Q, ld, T, ret, s_rate, nu_rate, PE, G, pending);
+  else if (noncentred) {
+    if (chunk <= 1) SV_POTENTIAL(1, true);
+    else if (chunk <= 2) SV_POTENTIAL(2, true);
+    else if (chunk <= 4) SV_POTENTIAL(4, true);
+    else if (chunk <= 6) SV_POTENTIAL(6, true);
+    else if (chunk <= 9) SV_POTENTIAL(9, true);
+    else if (chunk <= 12) SV_POTENTIAL(12, true);
+    else SV_POTENTIAL(16, true);
+  } else {
+    if (chunk <= 1) SV_POTENTIAL(1, false);
+    else if (chunk <= 2) SV_POTENTIAL(2, false);
+    else SV_POTENTIAL(4, false);
+  }
+#undef SV_POTENTIAL
+}
+
 cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, float* G, const int32_t* pending,
                              cudaStream_t st, bool fused_tick, bool dependent) {
   if (npts <= 0) return cudaSuccess;
@@ -406,8 +525,7 @@ cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, 
       break;
     }
     case 4:
-      sv_kernel<<<npts, 256, 0, st>>>(Q, npts, ld, (int)m.n, m.y, m.hyper[0], m.hyper[1], m.hyper[2] != 0.0, PE, G,
-                                      pending);
+      launch_sv(Q, npts, ld, (int)m.n, m.y, m.hyper[0], m.hyper[1], m.hyper[2] != 0.0, PE, G, pending, st);
       break;
     default:
       return cudaErrorInvalidValue;

@@ -295,4 +295,88 @@ __device__ __noinline__ void sv_nc_potential_block(const float* z, float* g, dou
   }
 }
 
+// ------------------------------------------------ eight element warps beside scalar warps
+// Pieces of the register engine (sv_engine.cuh) and of sv_potential_kernel: element thread i of 256, rows in shared
+// memory with one word more every 16, so that the non-centred walk's chunk order meets few bank conflicts.
+__device__ __forceinline__ int sv_pos(int d) { return d + (d >> 4); }
+
+// folds the eight warp sums of row i, as Group<256>::sumff
+__device__ __forceinline__ FF sv_fold(const float2 (*r)[8], int i) {
+  FF t{r[i][0].x, r[i][0].y};
+#pragma unroll
+  for (int w = 1; w < 8; ++w) t = ff_add(t, FF{r[i][w].x, r[i][w].y});
+  return t;
+}
+
+// block_excl_scan and block_excl_rscan over eight element warps (named barrier 2), one barrier each.
+__device__ __forceinline__ FF sv_excl_scan(FF v, int lane, int warp, float2* wt) {
+  FF excl{0.0f, 0.0f};
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    FF x{__shfl_up_sync(0xffffffffu, v.hi, o), __shfl_up_sync(0xffffffffu, v.lo, o)};
+    if (lane >= o) v = ff_add(x, v);
+  }
+  excl.hi = __shfl_up_sync(0xffffffffu, v.hi, 1);
+  excl.lo = __shfl_up_sync(0xffffffffu, v.lo, 1);
+  if (lane == 0) excl = FF{0.0f, 0.0f};
+  if (lane == 31) wt[warp] = make_float2(v.hi, v.lo);
+  asm volatile("bar.sync 2, 256;" ::: "memory");
+  FF off{0.0f, 0.0f};
+  for (int k = 0; k < warp; ++k) off = ff_add(off, FF{wt[k].x, wt[k].y});
+  return ff_add(off, excl);
+}
+__device__ __forceinline__ FF sv_excl_rscan(FF v, int lane, int warp, float2* wt) {
+  FF excl{0.0f, 0.0f};
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    FF x{__shfl_down_sync(0xffffffffu, v.hi, o), __shfl_down_sync(0xffffffffu, v.lo, o)};
+    if (lane + o < 32) v = ff_add(v, x);
+  }
+  excl.hi = __shfl_down_sync(0xffffffffu, v.hi, 1);
+  excl.lo = __shfl_down_sync(0xffffffffu, v.lo, 1);
+  if (lane == 31) excl = FF{0.0f, 0.0f};
+  if (lane == 0) wt[warp] = make_float2(v.hi, v.lo);
+  asm volatile("bar.sync 2, 256;" ::: "memory");
+  FF off{0.0f, 0.0f};
+  for (int k = 7; k > warp; --k) off = ff_add(off, FF{wt[k].x, wt[k].y});
+  return ff_add(off, excl);
+}
+
+// The non-centred walk's elements: gradients to gs (may be rets: a thread reads its chunk before it writes it), warp
+// sums of l1p, frac, h, a S and h_base^2 to r1.  K: steps a thread at most.  Steps past the chunk count as
+// zeros (adding 0 to a compensated sum changes nothing), so that the steps' long operations overlap.
+template <int K>
+__device__ __forceinline__ void sv_nc_elements(const float* zs, const float* rets, float* gs, int T, int tid, float sf,
+                                               float nuf, float inv_nuf, float2 (*r1)[8], float2 (*wt)[8]) {
+  const int lane = tid & 31, warp = tid >> 5;
+  const int chunk = (T + 255) / 256;
+  const int t0 = min(T, tid * chunk), t1 = min(T, t0 + chunk);
+  SvNcSums s{};
+  float av[K];
+  auto ev = [&](int i) -> float { return (t0 + i < t1) ? zs[sv_pos(t0 + i)] : 0.0f; };
+  Comp32 tot{0.0f, 0.0f};
+#pragma unroll
+  for (int i = 0; i < K; ++i) tot.add(ev(i));
+  const FF ck = sv_excl_scan(comp_ff(tot), lane, warp, wt[0]);
+  Comp32 S{ck.hi, ck.lo};
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const bool in = t0 + i < t1;
+    av[i] = sv_nc_step(S, ev(i), in ? rets[sv_pos(t0 + i)] : 0.0f, sf, nuf, inv_nuf, s, in);
+  }
+  const FF suf = sv_excl_rscan(comp_ff(s.atot), lane, warp, wt[1]);
+  Comp32 A{suf.hi, suf.lo};
+#pragma unroll
+  for (int i = K - 1; i >= 0; --i) {
+    A.add(av[i]);
+    if (t0 + i < t1) gs[sv_pos(t0 + i)] = ev(i) - sf * A.value();
+  }
+  const FF v = warp_sum4ff(comp_ff(s.l1p), comp_ff(s.frac), comp_ff(s.h), comp_ff(s.as), lane);
+  if ((lane & 7) == 0) r1[lane >> 3][warp] = make_float2(v.hi, v.lo);
+  FF e2 = comp_ff(s.e2);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e2 = ff_add(e2, ff_shfl_xor(e2, o));
+  if (lane == 0) r1[4][warp] = make_float2(e2.hi, e2.lo);
+}
+
 }  // namespace gbn
