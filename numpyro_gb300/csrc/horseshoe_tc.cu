@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_MISC);
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + OFF_MISC + NUM_BARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + OFF_MISC + NUM_BARS * 8 + 4);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * TN, m0 = blockIdx.y * TM;
   const int kb0 = blockIdx.z * G.kblocks_per_split;
   const int nkb = max(0, min(G.kblocks, kb0 + G.kblocks_per_split) - kb0);
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_holder;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_holder, 0);
   // B is the model's data: its first stages are on their way before the previous kernel (the state
   // machine, or GEMM1) has ended.  Everything else read here is that kernel's.
   auto load_b = [&](int i) {
@@ -190,9 +190,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    // The whole warp runs the loop and one elected lane issues each MMA and commit (issued by
-    // lane 0 alone, every tcgen05.mma paid a long issue latency); the stage descriptors are built
-    // once and moved by constant offsets.
+    // The whole warp runs the loop, on warp-uniform values, and one elected lane issues a K block's MMAs
+    // and commits (elect_one); the stage descriptors are built once and moved by constant offsets.
     constexpr uint32_t ID = idesc(TM, TN, 0, 0);  // both operands K-major
     constexpr int kPairA[NPAIRS] = {0, 0, 1, 0, 2, 1};
     constexpr int kPairB[NPAIRS] = {0, 1, 0, 2, 0, 1};
@@ -205,20 +204,26 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) hs_tc_gemm_kernel(const __grid
       tc_fence_after();
       const uint64_t st = sdesc_at(d0, (uint32_t)(s * STAGE_BYTES));
       const uint32_t at = tmem + A_COL + (uint32_t)hb * A_BUF;  // 8 columns per 16 of K
+      if (elect_one()) {
 #pragma unroll
-      for (int kk = 0; kk < TK / 16; ++kk)  // hh of this block into its own accumulator
-        mma_bf16_tmem_a_warp(tmem + (uint32_t)(hb * TN), at + kk * 8, sdesc_at(st, kk * 32), ID, kk > 0 ? 1u : 0u);
-      mma_commit_warp(hfull(hb));
-      // Corrections share one accumulator over the whole K range.  (Terms of B side by side in one MMA of 2 TN
-      // columns took a third fewer MMAs and 1.5 us off a tick, but sum the corrections in another order, and
-      // a trajectory of 32 leapfrog steps then ends 1e-4 elsewhere.)
-#pragma unroll
-      for (int p = 1; p < NPAIRS; ++p) {
-#pragma unroll
-        for (int kk = 0; kk < TK / 16; ++kk)
-          mma_bf16_tmem_a_warp(tmem + CORR_COL, at + kPairA[p] * A_TERM + kk * 8,
-                               sdesc_at(st, kPairB[p] * B_SPLIT + kk * 32), ID, (i > 0 || p > 1 || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < TK / 16; ++kk)  // hh of this block into its own accumulator
+          mma_bf16_tmem_a(tmem + (uint32_t)(hb * TN), at + kk * 8, sdesc_at(st, kk * 32), ID, kk > 0 ? 1u : 0u);
       }
+      __syncwarp();
+      mma_commit_warp(hfull(hb));
+      if (elect_one()) {
+        // Corrections share one accumulator over the whole K range.  (Terms of B side by side in one MMA of 2 TN
+        // columns took a third fewer MMAs and 1.5 us off a tick, but sum the corrections in another order, and
+        // a trajectory of 32 leapfrog steps then ends 1e-4 elsewhere.)
+#pragma unroll
+        for (int p = 1; p < NPAIRS; ++p) {
+#pragma unroll
+          for (int kk = 0; kk < TK / 16; ++kk)
+            mma_bf16_tmem_a(tmem + CORR_COL, at + kPairA[p] * A_TERM + kk * 8,
+                            sdesc_at(st, kPairB[p] * B_SPLIT + kk * 32), ID, (i > 0 || p > 1 || kk > 0) ? 1u : 0u);
+        }
+      }
+      __syncwarp();
       mma_commit_warp(empty(s));
       mma_commit_warp(aempty(hb));
     }

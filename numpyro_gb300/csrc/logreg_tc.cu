@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) logreg_tc_kernel(const __grid_
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + OFF_MISC + NUM_BARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + OFF_MISC + NUM_BARS * 8 + 4);
   double* ll_smem = reinterpret_cast<double*>(smem + OFF_MISC + 256);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int cb = blockIdx.x;  // chain block
   const int rg = blockIdx.y;  // row group
   const int64_t ntiles = (P.n + BM - 1) / BM;
@@ -320,9 +320,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) logreg_tc_kernel(const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_holder;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_holder, 0);
   const float lo2max = fmaxf(fmaxf(lo2_slot[0], lo2_slot[1]), fmaxf(lo2_slot[2], lo2_slot[3]));
-  const int nsplit = lo2max > P.lo2_limit ? 3 : 2;
+  const int nsplit = __shfl_sync(0xffffffffu, lo2max > P.lo2_limit ? 3 : 2, 0);
   if (threadIdx.x == 0 && rg == 0 && P.split3) P.split3[cb] = nsplit == 3 ? 1 : 0;
 
   if (warp == 0) {
@@ -351,10 +351,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) logreg_tc_kernel(const __grid_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    // The whole warp runs this loop and one elected lane issues each MMA and commit: from a
-    // converged warp the descriptor arithmetic stays warp-uniform.  (Run by lane 0 alone,
-    // each tcgen05.mma took ~70-90 cycles to issue and this loop, not the tensor pipe or the
-    // epilogue, set the tile rate.)  Descriptors are built once and moved by constant offsets.
+    // The whole warp runs this loop, on warp-uniform values, and one elected lane issues a GEMM's MMAs
+    // (elect_one).  This warp slows the four epilogue warps of one lane quadrant, on its scheduler, and the slowest
+    // quadrant sets the tile rate: with 19 instructions an MMA (an election, and descriptors moved to uniform
+    // registers) that scheduler issued 299,000 instructions where others had 227,000, now 261,000
+    // (0.223 -> 0.213 ms at 1024 chains x 581,012 rows).  An issuer per H buffer, on three schedulers, balanced
+    // the quadrants but was no faster (0.219 ms); H buffers of 64 rows were slower (0.28 ms: half as much per MMA).
+    // Descriptors are built once and moved by constant offsets.
     constexpr uint32_t ID1 = idesc(BN, BM, 0, 0);  // H = B . X'^T: chains x rows, both K-major
     constexpr uint32_t ID2 = idesc(BN, BK, 0, 1);  // G = E . X': E K-major in TMEM, X' MN-major
     const uint32_t xb = smem_u32(smem + OFF_X), bb = smem_u32(smem + OFF_B);
@@ -379,14 +382,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) logreg_tc_kernel(const __grid_
         tc_fence_after();
         const uint32_t d = tmem + (uint32_t)(bi * BM);
         const uint64_t xs = sdesc_at(dx1, (uint32_t)(si * X_TILE));
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < NSPLIT; ++k) {
-          if (k >= nsplit) break;
+          for (int k = 0; k < NSPLIT; ++k) {
+            if (k >= nsplit) break;
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk)
-            mma_bf16_warp(d, sdesc_at(dcoef, k * B_TILE + kk * 32), sdesc_at(xs, kk * 32), ID1,
-                          (k | kk) ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk)
+              mma_bf16(d, sdesc_at(dcoef, k * B_TILE + kk * 32), sdesc_at(xs, kk * 32), ID1, (k | kk) ? 1u : 0u);
+          }
         }
+        __syncwarp();
         mma_commit_warp(bar(B_ACCF + bi));
         if (++si == STAGES) si = 0, pi ^= 1;
         if (++bi == NBUF) bi = 0, qi ^= 1;
@@ -398,15 +403,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) logreg_tc_kernel(const __grid_
         tc_fence_after();
         const uint32_t ea = tmem + (uint32_t)(bj * BM);
         const uint64_t xs = sdesc_at(dx2, (uint32_t)(sj * X_TILE));
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < BM / 16; ++kk) {
-          // A = E rows 16kk..16kk+15: 8 TMEM columns in the block of the warp that wrote them
-          // (rows EPI_ROWS w + r at column EPI_ROWS w + r / 2); B = X' tile, MN-major (features
-          // contiguous), 8-row groups 1024 B apart
-          constexpr int KW = EPI_ROWS / 16;  // K steps per epilogue warp's block of rows
-          mma_bf16_tmem_a_warp(tmem + ACC2_COL, ea + (uint32_t)((kk / KW) * EPI_ROWS + (kk % KW) * 8),
-                               sdesc_at(xs, kk * 2048), ID2, (j > 0 || kk > 0) ? 1u : 0u);
+          for (int kk = 0; kk < BM / 16; ++kk) {
+            // A = E rows 16kk..16kk+15: 8 TMEM columns in the block of the warp that wrote them
+            // (rows EPI_ROWS w + r at column EPI_ROWS w + r / 2); B = X' tile, MN-major (features
+            // contiguous), 8-row groups 1024 B apart
+            constexpr int KW = EPI_ROWS / 16;  // K steps per epilogue warp's block of rows
+            mma_bf16_tmem_a(tmem + ACC2_COL, ea + (uint32_t)((kk / KW) * EPI_ROWS + (kk % KW) * 8),
+                            sdesc_at(xs, kk * 2048), ID2, (j > 0 || kk > 0) ? 1u : 0u);
+          }
         }
+        __syncwarp();
         mma_commit_warp(bar(B_SE + bj));
         mma_commit_warp(bar(B_XEMPTY + sj));
         if (++sj == STAGES) sj = 0;

@@ -1,7 +1,7 @@
 // tc_ptx.cuh -- inline-PTX building blocks of the tcgen05 kernels (logreg_tc.cu, horseshoe_tc.cu):
 // mbarriers with bounded waits (single thread and whole warp), TMA 2-D tile loads and L2
 // prefetches, shared-memory matrix descriptors, the kind::f16 instruction descriptor,
-// warp-issued tcgen05.mma / commit (A from shared memory or from TMEM), TMEM loads and stores,
+// tcgen05.mma / commit by an elected lane (A from shared memory or from TMEM), TMEM loads and stores,
 // and the approximate special functions of the logistic epilogue.
 #pragma once
 #include <cuda.h>
@@ -131,27 +131,36 @@ __host__ __device__ constexpr uint32_t idesc(int M, int N, int a_mn_major, int b
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn_major << 15) | ((uint32_t)b_mn_major << 16) |
          ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+// One lane of a converged warp (the same one every time).  The issuing warp runs its loop as a whole, with warp-uniform
+// values (its own index, the TMEM base and flags read from memory pass through __shfl_sync, which tells the
+// compiler so: descriptors then stay in uniform registers), and the elected lane issues a GEMM's MMAs
+// and commits.  Under `if (lane == 0)` an MMA took 70 to 90 cycles to issue; with an election per MMA and values
+// the compiler held for divergent it took 19 instructions, a third more than the scheduler's other warps had to do.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
 // tcgen05.mma (kind::f16, one CTA, D in TMEM, A and B from shared-memory descriptors; acc = 0
-// overwrites D), executed by a whole converged warp: one elected lane issues the MMA.  Issuing
-// from a converged warp keeps the descriptor arithmetic warp-uniform; from inside
-// `if (lane == 0)` every MMA cost ~70-90 cycles of issue latency.
-__device__ __forceinline__ void mma_bf16_warp(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
+// overwrites D), by the elected lane.
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\telect.sync _|e, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(a), "l"(b), "r"(id), "r"(acc)
       : "memory");
 }
-// As mma_bf16_warp with the A operand (M lanes x K, two bf16 per 32-bit column, the lower
+// As mma_bf16 with the A operand (M lanes x K, two bf16 per 32-bit column, the lower
 // half holding the even k) read from tensor memory at a_tmem instead of shared memory.
-__device__ __forceinline__ void mma_bf16_tmem_a_warp(uint32_t tmem_d, uint32_t a_tmem, uint64_t b, uint32_t id,
-                                                     uint32_t acc) {
+__device__ __forceinline__ void mma_bf16_tmem_a(uint32_t tmem_d, uint32_t a_tmem, uint64_t b, uint32_t id, uint32_t acc) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\telect.sync _|e, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
       "r"(a_tmem), "l"(b), "r"(id), "r"(acc)
       : "memory");
 }
+// The barrier's phase completes when the MMAs issued by the elected lane have (by the converged warp: commits inside
+// the elected lane's region were slower).
 __device__ __forceinline__ void mma_commit_warp(uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
