@@ -87,38 +87,39 @@ void logreg_prior_consts(double prior_scale, int p, float* inv_var_f, double* pe
 // Tiles of BM x 64 outputs, 4 x 8 a thread.  At 2000 x 1000 x 256 chains a GEMM has 512,000 outputs, under one
 // warp of 32 outputs a thread for each scheduler.  Bound: shared-memory reads (a 16-byte read of a warp takes
 // four cycles, broadcast or not, so 4 x 4 outputs a thread read 8 cycles for 4 of multiply-adds, 4 x 8 12
-// for 8).  cp.async runs HS_STAGES - 1 K steps ahead.
-constexpr int HS_BN = 64, HS_BK = 32, HS_STAGES = 2;
+// for 8).  cp.async runs STAGES - 1 K steps of BK ahead: 3 stages of 32 where the multiply-adds bound it (80 us a
+// potential at that size; 2 stages of 32 88, 4 of 16 85), 4 of 16 where a CTA has a few steps and their latency does
+// (542 x 130 x 3 chains: a run of 0.89 ms; 3 of 32 0.93, 2 of 32 0.95).
+constexpr int HS_BN = 64;
 constexpr int HS_SPLIT_ROWS = 16;  // a row range of the adjoint GEMM is a multiple of this
 constexpr int HS_MIN_BM = 32;     // smallest tile height offered to the tuner
 constexpr int HS_MAX_SPLITS = 8;  // most row ranges offered to the tuner for the adjoint GEMM
 
-template <int BM>
+template <int BM, int BK, int STAGES>
 __global__ void __launch_bounds__(BM * HS_BN / 32)
     hs_sgemm_nn_kernel(const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, int M, int N, int K,
                        int k_per_split, float* __restrict__ Out, int ldo, int64_t split_stride,
                        const float* __restrict__ yv, double* __restrict__ part_rr, int ld_rr, const int32_t* pending) {
   if (pending && *pending == 0) return;
   constexpr int NTH = BM * HS_BN / 32, TX = HS_BN / 8, TY = BM / 4;
-  __shared__ __align__(16) float As[HS_STAGES][HS_BK][BM];
-  __shared__ __align__(16) float Bs[HS_STAGES][HS_BK][HS_BN];
+  __shared__ __align__(16) float As[STAGES][BK][BM];
+  __shared__ __align__(16) float Bs[STAGES][BK][HS_BN];
   constexpr int SQ_ROWS = BM / 16;  // rows a sum of squares takes in FP32
-  __shared__ float rr[TY * 4 / SQ_ROWS][HS_BN];
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * HS_BN;
   const int kb = blockIdx.z * k_per_split, ke = min(K, kb + k_per_split);
-  const int steps = ke > kb ? (ke - kb + HS_BK - 1) / HS_BK : 0;
+  const int steps = ke > kb ? (ke - kb + BK - 1) / BK : 0;
   auto stage = [&](int step) {  // one K step of both operands; past the end an empty group
     if (step < steps) {
-      const int k0 = kb + step * HS_BK, s = step % HS_STAGES;
+      const int k0 = kb + step * BK, s = step % STAGES;
 #pragma unroll
-      for (int q = tid; q < HS_BK * BM / 4; q += NTH) {
+      for (int q = tid; q < BK * BM / 4; q += NTH) {
         const int k = q / (BM / 4), m = 4 * (q % (BM / 4));
         const bool in = k0 + k < ke && m0 + m < M;
         cp_async16(&As[s][k][m], in ? A + (size_t)(k0 + k) * lda + m0 + m : A, in);
       }
 #pragma unroll
-      for (int q = tid; q < HS_BK * HS_BN / 4; q += NTH) {
+      for (int q = tid; q < BK * HS_BN / 4; q += NTH) {
         const int k = q / (HS_BN / 4), n = 4 * (q % (HS_BN / 4));
         const bool in = k0 + k < ke && n0 + n < N;
         cp_async16(&Bs[s][k][n], in ? B + (size_t)(k0 + k) * ldb + n0 + n : B, in);
@@ -127,15 +128,15 @@ __global__ void __launch_bounds__(BM * HS_BN / 32)
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int i = 0; i < HS_STAGES - 1; ++i) stage(i);
+  for (int i = 0; i < STAGES - 1; ++i) stage(i);
   float acc[4][8] = {};
   for (int step = 0; step < steps; ++step) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(HS_STAGES - 2) : "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     __syncthreads();  // this step has landed, and every thread is done with the stage filled next
-    stage(step + HS_STAGES - 1);
-    const int s = step % HS_STAGES;
+    stage(step + STAGES - 1);
+    const int s = step % STAGES;
 #pragma unroll
-    for (int kk = 0; kk < HS_BK; ++kk) {
+    for (int kk = 0; kk < BK; ++kk) {
       const float4 a4 = *reinterpret_cast<const float4*>(&As[s][kk][4 * ty]);
       const float4 b4 = *reinterpret_cast<const float4*>(&Bs[s][kk][4 * tx]);
       const float4 c4 = *reinterpret_cast<const float4*>(&Bs[s][kk][HS_BN / 2 + 4 * tx]);
@@ -163,6 +164,8 @@ __global__ void __launch_bounds__(BM * HS_BN / 32)
     return;
   }
   // residual epilogue: R = y - acc, and per-chain sums of R^2 over this row tile
+  float(*const rr)[HS_BN] = reinterpret_cast<float(*)[HS_BN]>(&As[0][0][0]);  // [TY * 4 / SQ_ROWS], over the operands
+  __syncthreads();
   float sq[8] = {};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -509,17 +512,23 @@ cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, 
       hs_pack_kernel<<<gp, 256, 0, st>>>(Q, ld, npts, P, nc, m.hs_bt, cp, pp, pending);
       // R[row][c] = y[row] - sum_p X[row][p] beta_c[p]
       dim3 g1((npts + HS_BN - 1) / HS_BN, mt, 1);
+      auto gemm1 = [&](auto kernel, int threads) {
+        kernel<<<g1, threads, 0, st>>>(m.hs_xt, pad4(M), m.hs_bt, cp, M, npts, P, P, m.resid, cp, 0, m.y, m.part_rr, cp,
+                                       pending);
+      };
+      const bool large = npts >= 128 && m.n * P >= 1000000;  // as the tile height's rule (tune_params)
       if (tm == 2)
-        hs_sgemm_nn_kernel<32><<<g1, 64, 0, st>>>(m.hs_xt, pad4(M), m.hs_bt, cp, M, npts, P, P, m.resid, cp, 0, m.y,
-                                                  m.part_rr, cp, pending);
+        large ? gemm1(hs_sgemm_nn_kernel<32, 32, 3>, 64) : gemm1(hs_sgemm_nn_kernel<32, 16, 4>, 64);
       else
-        hs_sgemm_nn_kernel<64><<<g1, 128, 0, st>>>(m.hs_xt, pad4(M), m.hs_bt, cp, M, npts, P, P, m.resid, cp, 0, m.y,
-                                                   m.part_rr, cp, pending);
+        large ? gemm1(hs_sgemm_nn_kernel<64, 32, 3>, 128) : gemm1(hs_sgemm_nn_kernel<64, 16, 4>, 128);
       // GB[s][c][p] = sum_{row in split s} R[row][c] X[row][p]
       const int kps = (((M + splits - 1) / splits) + HS_SPLIT_ROWS - 1) / HS_SPLIT_ROWS * HS_SPLIT_ROWS;
       dim3 g2((P + HS_BN - 1) / HS_BN, (npts + 63) / 64, splits);
-      hs_sgemm_nn_kernel<64><<<g2, 128, 0, st>>>(m.resid, cp, m.hs_xp, pp, npts, P, M, kps, m.part_gb, pp,
-                                                 (int64_t)npts * pp, nullptr, nullptr, 0, pending);
+      auto gemm2 = [&](auto kernel) {
+        kernel<<<g2, 128, 0, st>>>(m.resid, cp, m.hs_xp, pp, npts, P, M, kps, m.part_gb, pp, (int64_t)npts * pp, nullptr,
+                                   nullptr, 0, pending);
+      };
+      large ? gemm2(hs_sgemm_nn_kernel<64, 32, 3>) : gemm2(hs_sgemm_nn_kernel<64, 16, 4>);
       horseshoe_finish_kernel<<<npts, 256, 0, st>>>(Q, npts, ld, P, m.n, m.part_gb, splits, pp, m.part_rr, cp, mt,
                                                     nc, PE, G, pending);
       break;
