@@ -641,7 +641,7 @@ def main():
                 "peak_kind": peak_kind + " burst bf16",
                 "kernel": ("logreg_tc_kernel (bf16x3; coefficient split and row-group finish fused into the "
                            "state-machine kernel)" if precision == "bf16x3" else
-                           "logreg potential (fp32: logreg_simt_kernel + logreg_finish_kernel)"),
+                           "logreg potential (fp32: logreg_fp32_kernel + logreg_fp32_finish_kernel)"),
                 "algorithmic_flop_per_launch": flop, "launch_ms": pot_ms}
     if precision == "bf16x3":
         # the special-function unit's share of the tensor-core potential (one ex2 per logit, tanh for
@@ -767,7 +767,7 @@ def _sfu_roofline(launch_ms, n, chains):
 def _launches_per_tick(precision):
     # advance_kernel, then the potential: on the tensor cores the tcgen05 kernel alone (the
     # coefficient split and the row-group finish run inside advance_kernel; GBN_FUSE_TICK=0 launches
-    # them separately, 4 per tick), on CUDA cores logreg_simt + logreg_finish
+    # them separately, 4 per tick), on CUDA cores logreg_fp32 + logreg_fp32_finish
     if precision == "bf16x3":
         return 4 if os.environ.get("GBN_FUSE_TICK", "1") == "0" else 2
     return 3
