@@ -92,8 +92,8 @@ void logreg_prior_consts(double prior_scale, int p, float* inv_var_f, double* pe
 // (542 x 130 x 3 chains: a run of 0.89 ms; 3 of 32 0.93, 2 of 32 0.95).
 constexpr int HS_BN = 64;
 constexpr int HS_SPLIT_ROWS = 16;  // a row range of the adjoint GEMM is a multiple of this
-constexpr int HS_MIN_BM = 32;     // smallest tile height offered to the tuner
-constexpr int HS_MAX_SPLITS = 8;  // most row ranges offered to the tuner for the adjoint GEMM
+constexpr int HS_MIN_BM = 32;     // smallest tile height; the partials are sized for it
+constexpr int HS_MAX_SPLITS = 8;  // most row ranges of the adjoint GEMM
 
 template <int BM, int BK, int STAGES>
 __global__ void __launch_bounds__(BM * HS_BN / 32)
