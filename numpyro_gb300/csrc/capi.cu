@@ -105,6 +105,7 @@ static int fail(gbn_handle h, int code, const std::string& msg) {
 
 static int cuda_fail(gbn_handle h, cudaError_t e, const char* what) {
   std::string msg = std::string(what) + ": " + cudaGetErrorString(e);
+  cudaGetLastError();  // reported here, and not again by the handle's next call
   return fail(h, GBN_ERR_CUDA, msg);
 }
 
@@ -745,15 +746,14 @@ int gbn_run(gbn_handle h, void* stream, gbn_state* st, int32_t num_iterations, i
     if (e != cudaSuccess) return cuda_fail(h, e, "gbn_run: queue");
     if (h->m.family == GBN_FAMILY_SV) {
       SvView sv{h->m.y, (int)h->m.n, h->m.hyper[2] != 0.0, h->m.hyper[0], h->m.hyper[1]};
-      launch_persistent_sv(h->dP, sv, h->counters + 7, h->C, h->D, h->cfg.algo == GBN_ALGO_NUTS,
-                           h->cfg.find_heuristic_step_size && h->cfg.adapt_step_size && h->num_warmup > 0, s);
+      e = launch_persistent_sv(h->dP, sv, h->counters + 7, h->C, h->D, h->cfg.algo == GBN_ALGO_NUTS,
+                               h->cfg.find_heuristic_step_size && h->cfg.adapt_step_size && h->num_warmup > 0, s);
     } else {
       HierView hv{h->m.y, h->m.hier_sinv, h->m.hier_cmodel, h->m.offsets, h->m.chains_per_model, h->m.num_models,
                   (float)(1.0 / (h->m.hyper[0] * h->m.hyper[0])), (float)(1.0 / h->m.hyper[1])};
-      launch_persistent_hier(h->dP, hv, h->counters + 7, h->order, h->C, h->D, h->maxd, h->cfg.algo == GBN_ALGO_NUTS,
-                             h->hp.dense != 0, s);
+      e = launch_persistent_hier(h->dP, hv, h->counters + 7, h->order, h->C, h->D, h->maxd,
+                                 h->cfg.algo == GBN_ALGO_NUTS, h->hp.dense != 0, s);
     }
-    e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(h, e, "gbn_run: persistent engine");
   } else {
@@ -844,19 +844,19 @@ int gbn_sample_async(gbn_handle h, void* stream, gbn_state* st) {
   if (h->persistent) {
     if (h->m.family == GBN_FAMILY_SV) {
       SvView sv{h->m.y, (int)h->m.n, h->m.hyper[2] != 0.0, h->m.hyper[0], h->m.hyper[1]};
-      launch_persistent_sv(h->dP, sv, h->counters + 7, h->C, h->D, h->cfg.algo == GBN_ALGO_NUTS,
-                           h->cfg.find_heuristic_step_size && h->cfg.adapt_step_size && h->num_warmup > 0, s);
+      e = launch_persistent_sv(h->dP, sv, h->counters + 7, h->C, h->D, h->cfg.algo == GBN_ALGO_NUTS,
+                               h->cfg.find_heuristic_step_size && h->cfg.adapt_step_size && h->num_warmup > 0, s);
     } else {
       HierView hv{h->m.y, h->m.hier_sinv, h->m.hier_cmodel, h->m.offsets, h->m.chains_per_model, h->m.num_models,
                   (float)(1.0 / (h->m.hyper[0] * h->m.hyper[0])), (float)(1.0 / h->m.hyper[1])};
-      launch_persistent_hier(h->dP, hv, h->counters + 7, h->order, h->C, h->D, h->maxd, h->cfg.algo == GBN_ALGO_NUTS,
-                             h->hp.dense != 0, s);
+      e = launch_persistent_hier(h->dP, hv, h->counters + 7, h->order, h->C, h->D, h->maxd,
+                                 h->cfg.algo == GBN_ALGO_NUTS, h->hp.dense != 0, s);
     }
   } else {
     e = cudaMemsetAsync(h->async_iter, 0, sizeof(int32_t), s);
     if (e == cudaSuccess) e = cudaGraphLaunch(h->async_graph, s);
-    if (e != cudaSuccess) return cuda_fail(h, e, "gbn_sample_async: launch");
   }
+  if (e != cudaSuccess) return cuda_fail(h, e, "gbn_sample_async: launch");
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(h, e, "gbn_sample_async");
   return GBN_OK;

@@ -27,6 +27,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "hier_potential.cuh"
@@ -1244,12 +1245,33 @@ __global__ void __launch_bounds__(256) persistent_sv_kernel(const AdvParams* __r
 }
 
 // --------------------------------------------------------------------- launchers
+// Raises a kernel's limit of dynamic shared memory to all that a block can have, once a device (done: its bits).
+// The limit belongs to the kernel on the device, so every handle shares it, and handles run from several threads:
+// set to the size of one launch, it could be lowered by another thread between that call and the launch.
+static cudaError_t raise_smem_limit(const void* kernel, std::atomic<uint64_t>& done, int dev, int optin) {
+  const uint64_t bit = dev < 64 ? uint64_t{1} << dev : 0;  // further devices: set again, to the same value
+  if (done.load() & bit) return cudaSuccess;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
+  if (e == cudaSuccess) done.fetch_or(bit);
+  return e;
+}
+
 // Shared memory of an SM for its chains' U-turn checkpoints (64, 96 and 180 KB: no faster).
 constexpr size_t HIER_CK_SMEM = 128 * 1024;
 
+static cudaError_t engine_device(int* dev, int* sms, int* optin) {
+  cudaError_t e = cudaGetDevice(dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, *dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, *dev);
+  return e;
+}
+
 template <int K, bool DM>
-static void launch_hier_reg(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order, int C,
-                            int D, int maxd, int sms, int optin, cudaStream_t st) {
+static cudaError_t launch_hier_reg(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order,
+                                   int C, int D, int maxd, int dev, int sms, int optin, cudaStream_t st) {
   // few chains: a warp per SM before any SM takes two
   const int warps = C <= sms ? 1 : (C <= 2 * sms || DM ? 2 : 4);
   const int resident = 12 / warps;  // CTAs per SM that the shared memory leaves room for
@@ -1259,53 +1281,45 @@ static void launch_hier_reg(const AdvParams* dP, const HierView& hv, int32_t* qu
   const size_t budget = std::min((size_t)(HIER_CK_SMEM / per_sm_needed), (size_t)optin - 2048 - mass);
   const int slots = (int)std::min((size_t)maxd, budget / slot);
   const size_t smem = slot * slots + mass;
-  cudaFuncSetAttribute(persistent_hier_reg_kernel<K, DM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static std::atomic<uint64_t> raised{0};
+  cudaError_t e = raise_smem_limit((const void*)persistent_hier_reg_kernel<K, DM>, raised, dev, optin);
+  if (e != cudaSuccess) return e;
   int blocks = need;
   if (need > sms) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_reg_kernel<K, DM>, 32 * warps, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_reg_kernel<K, DM>, 32 * warps, smem);
+    if (e != cudaSuccess) return e;
     blocks = std::min(need, sms * std::max(per_sm, 1));
   }
   persistent_hier_reg_kernel<K, DM><<<blocks, 32 * warps, smem, st>>>(dP, hv, queue_head, order, slots * 64 * K);
+  return cudaGetLastError();
 }
 
-void launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order,
-                            int C, int D, int maxd, bool nuts, bool dense, cudaStream_t st) {
+cudaError_t launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order,
+                                   int C, int D, int maxd, bool nuts, bool dense, cudaStream_t st) {
   int dev = 0, sms = 0, per_sm = 0, optin = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaError_t e = engine_device(&dev, &sms, &optin);
+  if (e != cudaSuccess) return e;
   // The register engine holds up to 288 dimensions (nine elements a lane), 96 with a dense mass matrix (in
   // shared memory, up to 36 KB a chain); HMC and larger models run the state machine over memory.
-#define HIER_REG(K, DM) launch_hier_reg<K, DM>(dP, hv, queue_head, order, C, D, maxd, sms, optin, st)
+#define HIER_REG(K, DM) launch_hier_reg<K, DM>(dP, hv, queue_head, order, C, D, maxd, dev, sms, optin, st)
   if (nuts && D <= (dense ? 96 : 288)) {
     if (dense) {
-      if (D <= 32)
-        HIER_REG(1, true);
-      else if (D <= 64)
-        HIER_REG(2, true);
-      else
-        HIER_REG(3, true);
-    } else if (D <= 32) {
-      HIER_REG(1, false);
-    } else if (D <= 64) {
-      HIER_REG(2, false);
-    } else if (D <= 96) {
-      HIER_REG(3, false);
-    } else if (D <= 160) {
-      HIER_REG(5, false);
-    } else if (D <= 224) {
-      HIER_REG(7, false);
-    } else {
-      HIER_REG(9, false);
+      if (D <= 32) return HIER_REG(1, true);
+      if (D <= 64) return HIER_REG(2, true);
+      return HIER_REG(3, true);
     }
-    return;
+    if (D <= 32) return HIER_REG(1, false);
+    if (D <= 64) return HIER_REG(2, false);
+    if (D <= 96) return HIER_REG(3, false);
+    if (D <= 160) return HIER_REG(5, false);
+    if (D <= 224) return HIER_REG(7, false);
+    return HIER_REG(9, false);
   }
 #undef HIER_REG
-  if (dense)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_kernel<true>, 256, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_hier_kernel<false>, 256, 0);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per_sm, dense ? persistent_hier_kernel<true> : persistent_hier_kernel<false>, 256, 0);
+  if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   int blocks = sms * per_sm;
   int need = (C + 7) / 8;  // never more warps than chains
@@ -1314,54 +1328,46 @@ void launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* qu
     persistent_hier_kernel<true><<<blocks, 256, 0, st>>>(dP, hv, queue_head, order);
   else
     persistent_hier_kernel<false><<<blocks, 256, 0, st>>>(dP, hv, queue_head, order);
+  return cudaGetLastError();
 }
 
 template <int K, bool NC>
-static void launch_sv_reg(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, int sms,
-                          cudaStream_t st) {
+static cudaError_t launch_sv_reg(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, int dev,
+                                 int sms, int optin, cudaStream_t st) {
   const size_t smem = sv_engine_smem(D, NC, K);
-  cudaFuncSetAttribute(persistent_sv_reg_kernel<K, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static std::atomic<uint64_t> raised{0};
+  cudaError_t e = raise_smem_limit((const void*)persistent_sv_reg_kernel<K, NC>, raised, dev, optin);
+  if (e != cudaSuccess) return e;
   int blocks = C;
   if (C > sms) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_sv_reg_kernel<K, NC>, 320, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_sv_reg_kernel<K, NC>, 320, smem);
+    if (e != cudaSuccess) return e;
     blocks = std::min(C, sms * std::max(per_sm, 1));
   }
   persistent_sv_reg_kernel<K, NC><<<blocks, 320, smem, st>>>(dP, sv, queue_head);
-}
-template <int K>
-static void launch_sv_reg(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, int sms,
-                          cudaStream_t st) {
-  if (sv.noncentred)
-    launch_sv_reg<K, true>(dP, sv, queue_head, C, D, sms, st);
-  else
-    launch_sv_reg<K, false>(dP, sv, queue_head, C, D, sms, st);
+  return cudaGetLastError();
 }
 
-void launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, bool nuts,
-                          bool searches, cudaStream_t st) {
+cudaError_t launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, bool nuts,
+                                 bool searches, cudaStream_t st) {
   int dev = 0, sms = 0, per_sm = 0, optin = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaError_t e = engine_device(&dev, &sms, &optin);
+  if (e != cudaSuccess) return e;
   // The on-chip engine holds 17 coordinates a thread (4,352); HMC, longer walks and warmup with step-size
   // searches run the state machine over memory.
   if (nuts && !searches && D <= 4352 && (!sv.noncentred || sv.T <= 4096)) {
-    if (D <= 256)
-      launch_sv_reg<1>(dP, sv, queue_head, C, D, sms, st);
-    else if (D <= 512)
-      launch_sv_reg<2>(dP, sv, queue_head, C, D, sms, st);
-    else if (D <= 1024)
-      launch_sv_reg<4>(dP, sv, queue_head, C, D, sms, st);
-    else if (D <= 1536)
-      launch_sv_reg<6>(dP, sv, queue_head, C, D, sms, st);
-    else if (D <= 2304)
-      launch_sv_reg<9>(dP, sv, queue_head, C, D, sms, st);
-    else if (D <= 3328)
-      launch_sv_reg<13>(dP, sv, queue_head, C, D, sms, st);
-    else
-      launch_sv_reg<17>(dP, sv, queue_head, C, D, sms, st);
-    return;
+#define SV_REG(K)                                                                            \
+  (sv.noncentred ? launch_sv_reg<K, true>(dP, sv, queue_head, C, D, dev, sms, optin, st) \
+                 : launch_sv_reg<K, false>(dP, sv, queue_head, C, D, dev, sms, optin, st))
+    if (D <= 256) return SV_REG(1);
+    if (D <= 512) return SV_REG(2);
+    if (D <= 1024) return SV_REG(4);
+    if (D <= 1536) return SV_REG(6);
+    if (D <= 2304) return SV_REG(9);
+    if (D <= 3328) return SV_REG(13);
+    return SV_REG(17);
+#undef SV_REG
   }
   // On-chip rows make each leaf about a quarter faster (T = 4096 on GB300), but at 12 D floats per
   // CTA they can cost resident chains (197 KB: one CTA per SM, against two with global rows).  They
@@ -1369,11 +1375,15 @@ void launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t* queue_
   const size_t onchip = sizeof(float) * (size_t)SV_ONCHIP_VECS * D;
   bool use_onchip = onchip + sizeof(SvSmem<256>) + 64 <= (size_t)optin;
   if (use_onchip) {
-    cudaFuncSetAttribute(persistent_sv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)onchip);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_sv_kernel<true>, 256, onchip);
+    static std::atomic<uint64_t> raised{0};
+    e = raise_smem_limit((const void*)persistent_sv_kernel<true>, raised, dev, optin);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_sv_kernel<true>, 256, onchip);
+    if (e != cudaSuccess) return e;
     if (per_sm < 1 || (int64_t)sms * per_sm < C) use_onchip = false;
   }
-  if (!use_onchip) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_sv_kernel<false>, 256, 0);
+  if (!use_onchip) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_sv_kernel<false>, 256, 0);
+  if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   int blocks = sms * per_sm;
   if (blocks > C) blocks = C;
@@ -1381,6 +1391,7 @@ void launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t* queue_
     persistent_sv_kernel<true><<<blocks, 256, onchip, st>>>(dP, sv, queue_head);
   else
     persistent_sv_kernel<false><<<blocks, 256, 0, st>>>(dP, sv, queue_head);
+  return cudaGetLastError();
 }
 
 void launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity, cudaStream_t st,
