@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(256) sv_nc_long_kernel(const float* __restrict
   if (pending && *pending == 0) return;
   __shared__ SvSmem<256> sm;
   const size_t c = blockIdx.x;
-  sv_nc_potential_block<256>(Q + c * ld, G + c * ld, PE + c, T, ret, s_rate, nu_rate, threadIdx.x, sm);
+  sv_nc_potential_block<256, 8>(Q + c * ld, G + c * ld, PE + c, T, ret, s_rate, nu_rate, threadIdx.x, sm);
 }
 
 // CTA per point: eight element warps, and two scalar warps for what is FP64 or long (on GB300 a log-gamma takes
