@@ -102,11 +102,21 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
     };
     if (DM) {  // M^-1 may have changed at a window end
       const float* const src = P.s.inverse_mass_matrix + row * P.D;
+      constexpr int B = 8;  // rows in flight: one at a time, 96 rows took 33 us, half of a transition of one leaf
       __syncwarp();
-      for (int j = 0; j < D; ++j)
+      for (int j = 0; j < D; j += B) {
+        float a[B][K];
 #pragma unroll
-        for (int k = 0; k < K; ++k)
-          minv[j * (32 * K) + 32 * k + lane] = lane + 32 * k < D ? src[(size_t)j * P.D + lane + 32 * k] : 0.0f;
+        for (int i = 0; i < B; ++i)
+#pragma unroll
+          for (int k = 0; k < K; ++k)
+            a[i][k] = j + i < D && lane + 32 * k < D ? src[(size_t)(j + i) * P.D + lane + 32 * k] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < B; ++i)
+#pragma unroll
+          for (int k = 0; k < K; ++k)
+            if (j + i < D) minv[(j + i) * (32 * K) + 32 * k + lane] = a[i][k];
+      }
       __syncwarp();
     }
 #pragma unroll
