@@ -13,8 +13,9 @@
 // Measured at 581,012 x 55 x 1,024 chains: 5.52 ms (64 x 64 tile, 4 x 4 a thread, X through registers and a
 // transposed copy) -> 3.64 ms = 36 TFLOP/s.  8 x 8 logits a thread with 8 warps per SM: 3.85; scalar
 // multiply-adds: 3.86.
-// Sums: a chain's log-likelihood of four consecutive rows in FP32, then compensated FP32 over the
-// thread's rows and float-float across threads; FP64 across CTAs.
+// Sums: a chain's log-likelihood of four consecutive rows in FP32, then FP64 over the thread's rows, across threads
+// and across CTAs.  (Compensated FP32 pairs within a CTA leave the potential 2^-48 off instead of 2^-53 and are
+// 3 % faster at 5 features, 1.72 against 1.78 ms at 581,012 x 1,024; at 55 features both take 3.68.)
 #pragma once
 #include <algorithm>
 
@@ -62,7 +63,7 @@ template <int CT, int NTH, int RG, int CG, int FG, int SP, int NB>
 struct LogregTile {
   static constexpr int TX = CT / (4 * CG), TY = NTH / TX, RT = 4 * RG * TY;
   static constexpr size_t bytes(int dp) {
-    return sizeof(float) * (size_t)(NB * RT * SP + dp * CT + RT * CT + NB * RT) + sizeof(float2) * (NTH / 32) * CT;
+    return sizeof(float) * (size_t)(NB * RT * SP + dp * CT + RT * CT + NB * RT) + sizeof(double) * (NTH / 32) * CT;
   }
 };
 
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
   float* const xs = lr_smem;                 // [NB][RT][SP], chunk c of row r at c ^ ((r >> 2) & 7)
   float* const es = xs + NB * RT * SP;       // [RT][CT]
   float* const ys = es + RT * CT;            // [NB][RT]
-  float2* const lls = reinterpret_cast<float2*>(ys + NB * RT);  // [NTH / 32][CT]
+  double* const lls = reinterpret_cast<double*>(ys + NB * RT);  // [NTH / 32][CT]
   float* const bs = reinterpret_cast<float*>(lls + (NTH / 32) * CT);  // [4 nc][CT]
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int c0 = blockIdx.x * CT, rg = blockIdx.y, groups = gridDim.y;
@@ -123,9 +124,9 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
   for (int i = 0; i < 2 * CG; ++i)
 #pragma unroll
     for (int j = 0; j < 4 * FG; ++j) gacc[i][j] = make_float2(0.0f, 0.0f);
-  Comp32 ll[4 * CG];
+  double ll[4 * CG];
 #pragma unroll
-  for (int j = 0; j < 4 * CG; ++j) ll[j] = Comp32{0.0f, 0.0f};
+  for (int j = 0; j < 4 * CG; ++j) ll[j] = 0.0;
 
   int buf = 0;
   if (rg < ntiles) load_tile(rg, 0);
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
               make_float4(ev[4 * h], ev[4 * h + 1], ev[4 * h + 2], ev[4 * h + 3]);
       }
 #pragma unroll
-      for (int j = 0; j < 4 * CG; ++j) ll[j].add(llt[j]);
+      for (int j = 0; j < 4 * CG; ++j) ll[j] += f2d(llt[j]);
     }
     __syncthreads();
     // ------------------------------------------------ gradient
@@ -252,16 +253,16 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
   }
 #pragma unroll
   for (int j = 0; j < 4 * CG; ++j) {
-    FF v = comp_ff(ll[j]);
+    double v = ll[j];
 #pragma unroll
-    for (int o = 16; o >= TX; o >>= 1) v = ff_add(v, ff_shfl_xor(v, o));
-    if ((tid & 31) < TX) lls[(tid >> 5) * CT + (j >> 2) * (CT / CG) + 4 * tx + (j & 3)] = make_float2(v.hi, v.lo);
+    for (int o = 16; o >= TX; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((tid & 31) < TX) lls[(tid >> 5) * CT + (j >> 2) * (CT / CG) + 4 * tx + (j & 3)] = v;
   }
   __syncthreads();
   if (tid < CT && c0 + tid < A.npts) {
-    FF v{lls[tid].x, lls[tid].y};
-    for (int w = 1; w < NTH / 32; ++w) v = ff_add(v, FF{lls[w * CT + tid].x, lls[w * CT + tid].y});
-    A.part_ll[(size_t)rg * A.npts + c0 + tid] = ff_value(v);
+    double v = lls[tid];
+    for (int w = 1; w < NTH / 32; ++w) v += lls[w * CT + tid];
+    A.part_ll[(size_t)rg * A.npts + c0 + tid] = v;
   }
 }
 
