@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
               make_float4(ev[4 * h], ev[4 * h + 1], ev[4 * h + 2], ev[4 * h + 3]);
       }
 #pragma unroll
-      for (int j = 0; j < 4 * CG; ++j) ll[j] += f2d(llt[j]);
+      for (int j = 0; j < 4 * CG; ++j) ll[j] = CT <= 16 && tile == rg ? f2d(llt[j]) : ll[j] + f2d(llt[j]);  // few-chain tiles: no addition of 0
     }
     __syncthreads();
     // ------------------------------------------------ gradient
@@ -251,12 +251,33 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
       }
     }
   }
+  // Across the lanes of a warp that share chains.  An SM starts an FP64 instruction every 19 cycles, so the lanes first
+  // deal the 4 CG sums out among themselves (lane bit o set: the upper half of those left).
+  int left_sums = 4 * CG, first = 0, whole = 0;
 #pragma unroll
-  for (int j = 0; j < 4 * CG; ++j) {
-    double v = ll[j];
+  for (int o = 16; o >= TX; o >>= 1) {
+    if (left_sums > 1) {
+      left_sums >>= 1;
+      const bool up = (tid & o) != 0;
+      if (up) first += left_sums;
 #pragma unroll
-    for (int o = 16; o >= TX; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((tid & 31) < TX) lls[(tid >> 5) * CT + (j >> 2) * (CT / CG) + 4 * tx + (j & 3)] = v;
+      for (int j = 0; j < 2 * CG; ++j) {
+        if (j >= left_sums) break;
+        const double lower = ll[j], upper = ll[j + left_sums];
+        ll[j] = (up ? upper : lower) + __shfl_xor_sync(0xffffffffu, up ? lower : upper, o);
+      }
+    } else {
+      ll[0] += __shfl_xor_sync(0xffffffffu, ll[0], o);
+      whole |= o;
+    }
+  }
+  if ((tid & whole) == 0) {
+#pragma unroll
+    for (int k = 0; k < 2 * CG; ++k) {
+      if (k >= left_sums) break;
+      const int j = first + k;
+      lls[(tid >> 5) * CT + (j >> 2) * (CT / CG) + 4 * tx + (j & 3)] = ll[k];
+    }
   }
   __syncthreads();
   if (tid < CT && c0 + tid < A.npts) {
