@@ -214,9 +214,10 @@ int gbn_run(gbn_handle h, void* stream, gbn_state* st, int32_t num_iterations,
 
 int gbn_get_stats(gbn_handle h, gbn_stats* stats);
 /* Launch shapes the autotuner chose at gbn_create for this model's potential kernels ("name=value ...",
- * empty when nothing was tuned).  The autotuner times the candidate chains-per-CTA and row-group shapes
- * once per process for each (device, model shape, chain count); GBN_AUTOTUNE=0 in the environment
- * keeps the defaults.  The horseshoe's tile rows and splits follow a rule on its sizes.  No counterpart in the reference. */
+ * empty when nothing was tuned).  The autotuner times the candidate chains-per-CTA shapes of the hierarchical
+ * kernel, which do not change a result, once per process for each (device, model shape, chain count);
+ * GBN_AUTOTUNE=0 in the environment keeps the default.  The logistic kernel's row groups and the horseshoe's
+ * tile rows and splits set the order of FP32 sums and follow rules on the sizes.  No counterpart in the reference. */
 const char* gbn_tuning(gbn_handle h);
 
 /* Measurement utility, no counterpart in the reference: the mean CUDA-event time (ms) of `reps`

@@ -8,10 +8,10 @@ namespace gbn {
 
 struct AdvParams;
 
-// Launch shapes of the potential kernels, chosen by autotune_potential (defaults before tuning).
-// hier_cpb: chains (warps) per CTA of the hierarchical kernel; hs_tm: rows per thread of the horseshoe
+// Launch shapes of the potential kernels, chosen by autotune_potential (defaults before tuning) where they do not
+// change a result's bits, else by rule.  hier_cpb: chains (warps) per CTA of the hierarchical kernel; hs_tm: rows per thread of the horseshoe
 // residual GEMM (tile height 16 * hs_tm); hs_splits: row ranges of the horseshoe adjoint GEMM;
-// lr_rg: row groups of the FP32 logistic kernel (0: the allocation default).
+// lr_rg: row groups of the FP32 logistic kernel (0: by rule, logreg_fp32_row_groups).
 struct TuneParams {
   int hier_cpb = 8;
   int hs_tm = 4;
@@ -36,7 +36,7 @@ struct ModelDev {
   // scratch (sized for scratch_points potential points)
   TuneParams tune;
   int scratch_points = 0;
-  int row_groups = 0;       // default row groups of the FP32 logistic kernel
+  int row_groups = 0;       // row groups of the logistic kernel: the FP32 one's, at most so many of the tensor-core one
   int row_groups_cap = 0;   // row groups the logistic partial buffers hold
   float* part_g = nullptr;    // [row_groups][points][64]
   double* part_ll = nullptr;  // [row_groups][points]

@@ -370,13 +370,13 @@ cudaError_t ensure_potential_scratch(ModelDev& m, int points) {
   free_potential_scratch(m);
   cudaError_t e = cudaSuccess;
   if (m.family == 2) {
-    // Partials for the row groups of both kernels: the tensor-core one takes at most 152 over its blocks of
-    // 128 chains, the FP32 one its default, with room for the tuner to try twice as many.
-    const int64_t ntiles = (m.n + 63) / 64;
-    const int tc_rg = (int)std::min<int64_t>(std::max(1, 152 / ((points + 127) / 128)), ntiles);
-    const int rg = logreg_fp32_row_groups(m.n, points, 0);
-    m.row_groups = std::max(tc_rg, rg);
-    m.row_groups_cap = (int)std::min<int64_t>(std::max<int64_t>(m.row_groups, 2 * (int64_t)rg), ntiles);
+    // Partials: the FP32 kernel's row groups follow its rule, the tensor-core one takes at most 4 x 152 over blocks
+    // of 64 chains (it has blocks of 128 and 152 CTAs, more only for fewer points than these); GBN_TUNE may ask
+    // for twice as many.
+    const int64_t ntiles = (m.n + 63) / 64, blocks = (points + 63) / 64;
+    m.row_groups = m.tc ? (int)std::min<int64_t>((4 * 152 + blocks - 1) / blocks, ntiles)
+                        : logreg_fp32_row_groups(m.n, m.p, points, 0);
+    m.row_groups_cap = (int)std::min<int64_t>(2 * (int64_t)m.row_groups, ntiles);
     if (m.tune.lr_rg > m.row_groups_cap) m.tune.lr_rg = 0;
     e = cudaMalloc(&m.part_g, sizeof(float) * (size_t)m.row_groups_cap * points * 64);
     if (e == cudaSuccess) e = cudaMalloc(&m.part_ll, sizeof(double) * (size_t)m.row_groups_cap * points);
@@ -492,9 +492,9 @@ cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, 
       break;
     case 2: {
       if (m.precision == 1 && m.tc) return logreg_tc_launch(m, Q, npts, PE, G, pending, st, fused_tick);
-      // the tuned row groups belong to the handle's own number of points; the partials bound any other
+      // forced row groups belong to the handle's own number of points; the partials bound any other
       const int want = npts == m.scratch_points ? m.tune.lr_rg : 0;
-      const int rg = (int)std::min<int64_t>(logreg_fp32_row_groups(m.n, npts, want),
+      const int rg = (int)std::min<int64_t>(logreg_fp32_row_groups(m.n, m.p, npts, want),
                                             (int64_t)m.row_groups_cap * m.scratch_points / npts);
       e = launch_logreg_fp32(m.x, m.y, m.n, m.p, m.hyper[0], Q, npts, ld, rg, m.part_g, m.part_ll, PE, G, pending, st,
                              dependent);
@@ -615,17 +615,6 @@ cudaError_t autotune_potential(ModelDev& m, const float* Q, int npts, double* PE
         t.hier_cpb = cpb;
         cand.push_back(t);
       }
-    } else if (m.family == 2 && !(m.precision == 1 && m.tc)) {
-      const int rg0 = logreg_fp32_row_groups(m.n, npts, 0);
-      if (m.n <= 64 * LR_ORDERED) {  // one row group a tile
-        t.lr_rg = rg0;
-        cand.push_back(t);
-      } else {
-        for (int rg : {std::max(1, rg0 / 2), rg0, std::min(2 * rg0, m.row_groups_cap)}) {
-          t.lr_rg = logreg_fp32_row_groups(m.n, npts, rg);
-          cand.push_back(t);
-        }
-      }
     } else if (m.family == 3) {
       // By rule, not by timing: both shapes set the order of FP32 sums, and a choice made by a few
       // launches' times made a model's results differ between processes.
@@ -740,7 +729,7 @@ namespace gbn {
 cudaError_t launch_logreg_simt_scratch(const float* x, const float* y, int64_t n, int p, double prior_scale,
                                        const float* Q, int npts, int row_groups, float* part_g, double* part_ll,
                                        double* PE, float* G, cudaStream_t st) {
-  return launch_logreg_fp32(x, y, n, p, prior_scale, Q, npts, p, logreg_fp32_row_groups(n, npts, row_groups), part_g,
+  return launch_logreg_fp32(x, y, n, p, prior_scale, Q, npts, p, logreg_fp32_row_groups(n, p, npts, row_groups), part_g,
                             part_ll, PE, G, nullptr, st, false);
 }
 
