@@ -18,6 +18,7 @@
 // 3 % faster at 5 features, 1.72 against 1.78 ms at 581,012 x 1,024; at 55 features both take 3.68.)
 #pragma once
 #include <algorithm>
+#include <climits>
 
 #include "common.cuh"
 #include "internal.h"
@@ -287,12 +288,19 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
   }
 }
 
-// Row tiles of 64 rows: up to this many, every tile is a row group of its own and the finish adds them in
-// order, so a small data set's gradient is one fixed sum whatever the launch shape.
+// Row tiles of 64 rows: up to this many, for LR_ORDERED_POINTS points at most, every tile is a row group of its
+// own and the finish adds them in order, so a small data set's gradient is one fixed sum whatever the launch
+// shape.  More points would make the partials large (128 groups x 65,536 points: 2.2 GB) and their sum slow:
+// 1,000 rows x 5 features x 65,536 points 492 us, 283 with two groups.
 constexpr int LR_ORDERED = 128;
+constexpr int LR_ORDERED_POINTS = 1024;
 
 // The sums over row groups and the prior for one chain, a CTA of 256 threads.  By one warp the loads of
-// ~150 row groups (a few-chain launch) took 29 us in dependent rounds of eight.
+// ~150 row groups (a few-chain launch) took 29 us in dependent rounds of eight.  Where CTAs come in waves, or
+// a warp has two such rounds, a warp a chain (logreg_finish_kernel, the same order up to LR_ORDERED row groups)
+// is better: 200 rows x 16,384 points 76 against 45 us, x 1,024 16.4 against 14.4; 8,192 rows (128 groups) x
+// 1,024 points of 55 features 97 against 104.
+inline bool logreg_fp32_finish_by_warp(int npts, int groups) { return npts > 1024 || (npts > 512 && groups <= 16); }
 __global__ void __launch_bounds__(256) logreg_fp32_finish_kernel(const LogregArgs A, int groups, float inv_var,
                                                                  double pe_const, double* __restrict__ pe,
                                                                  float* __restrict__ g) {
@@ -351,15 +359,17 @@ constexpr int LR_SMS = 152;
 struct LogregShape {
   int variant, ct;
 };
-inline LogregShape logreg_fp32_shape(int64_t n, int npts) {
-  const int64_t tiles = (n + 63) / 64;
+// max_groups: row groups that the caller has room for (16 of 20,000 rows x 256 points x 55 features: 183 us with the
+// tile of 128 chains, 117 with 64, 99 with 16)
+inline LogregShape logreg_fp32_shape(int64_t n, int npts, int max_groups) {
+  const int64_t tiles = std::min<int64_t>((n + 63) / 64, max_groups);
   if (npts > 64 && (npts + 127) / 128 * tiles >= 2 * LR_SMS) return {3, 128};
   if (npts > 16 && (npts + 63) / 64 * tiles >= LR_SMS) return {2, 64};
   if (npts > 8) return {1, 16};
   return {0, 8};
 }
 // Row groups (CTAs of a chain group) by a rule on the sizes, as they set the order of FP32 sums: picked by timing, a
-// model's draws differed between processes.  One a tile for small data sets, else the same number of tiles in
+// model's draws differed between processes.  One a tile for small data sets of up to LR_ORDERED_POINTS points, else the same number of tiles in
 // every group where that can be, and of the counts that put k = 1 to 8 CTAs on the busiest SM the largest (with
 // the shortest sums) within 1 % of the least cost:
 //   k (tiles of a CTA + 0.15) f + 0.004 for each group (the finish),
@@ -369,9 +379,10 @@ inline LogregShape logreg_fp32_shape(int64_t n, int npts) {
 // Over 900 shapes of 8,193 to 581,012 rows, 5 to 55 features and 1 to 1,024 chains this is 0.5 % slower on average than
 // the best of up to 20 group counts (the best of three timed ones, as before: 1.8 %).  want > 0: at most that many.
 inline int logreg_fp32_row_groups(int64_t n, int p, int npts, int want) {
-  const LogregShape s = logreg_fp32_shape(n, npts);
   const int64_t tiles = (n + 63) / 64;
-  if (tiles <= LR_ORDERED) return (int)(want > 0 ? std::min<int64_t>(want, tiles) : tiles);
+  if (tiles <= LR_ORDERED && want > 0) return (int)std::min<int64_t>(want, tiles);
+  if (tiles <= LR_ORDERED && npts <= LR_ORDERED_POINTS) return (int)tiles;
+  const LogregShape s = logreg_fp32_shape(n, npts, INT_MAX);
   const int cgroups = (npts + s.ct - 1) / s.ct;
   auto even = [&](int64_t groups) {  // the same number of tiles each
     const int64_t g = std::min<int64_t>(std::max<int64_t>(groups, 1), tiles), per = (tiles + g - 1) / g;

@@ -55,13 +55,15 @@ __global__ void __launch_bounds__(512) hier_nc_kernel(const float* __restrict__ 
 }
 
 // ============================================================ logistic regression
-// sum the tensor-core kernel's partials, add the N(0, scale) prior; warp per point
+// sum the tensor-core kernel's partials, or the FP32 one's of many points, add the N(0, scale) prior; warp per point
 // lin (FP64 [p]): a linear term lin . b of the log-likelihood computed outside the kernel
 __global__ void logreg_finish_kernel(const float* __restrict__ Q, int npts, int ld, int p, int row_groups,
                                      const float* __restrict__ part_g, const double* __restrict__ part_ll,
                                      const double* __restrict__ lin, float inv_var_f, double pe_const,
                                      double* __restrict__ PE, float* __restrict__ G, const int32_t* pending,
                                      const int32_t* __restrict__ split3 = nullptr, bool e_tanh = false) {
+  tick_wait();
+  tick_trigger();
   if (pending && *pending == 0) return;
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c >= npts) return;
@@ -435,18 +437,21 @@ cudaError_t logreg_simt_smem_attr() {
   return e;
 }
 
-static cudaError_t launch_logreg_fp32(const float* x, const float* y, int64_t n, int p, double prior_scale,
+static cudaError_t launch_logreg_fp32(int variant, const float* x, const float* y, int64_t n, int p, double prior_scale,
                                       const float* Q, int npts, int ld, int row_groups, float* part_g, double* part_ll,
                                       double* PE, float* G, const int32_t* pending, cudaStream_t st,
                                       bool dependent) {
   cudaError_t e = logreg_simt_smem_attr();
   if (e != cudaSuccess) return e;
   const LogregArgs A{x, y, n, p, Q, npts, ld, part_g, part_ll, pending};
-  e = logreg_fp32_launch(logreg_fp32_shape(n, npts).variant, A, row_groups, st, dependent);
+  e = logreg_fp32_launch(variant, A, row_groups, st, dependent);
   if (e != cudaSuccess) return e;  // checked per launch, so the first failing launch is the one reported
   float ivf;
   double pec;
   logreg_prior_consts(prior_scale, p, &ivf, &pec);
+  if (logreg_fp32_finish_by_warp(npts, row_groups))
+    return launch_tick(logreg_finish_kernel, (npts + 7) / 8, 256, 0, st, dependent, Q, npts, ld, p, row_groups, part_g,
+                       part_ll, nullptr, ivf, pec, PE, G, pending, nullptr, false);
   return launch_tick(logreg_fp32_finish_kernel, npts, 256, 0, st, dependent, A, row_groups, ivf, pec, PE, G);
 }
 
@@ -496,8 +501,8 @@ cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, 
       const int want = npts == m.scratch_points ? m.tune.lr_rg : 0;
       const int rg = (int)std::min<int64_t>(logreg_fp32_row_groups(m.n, m.p, npts, want),
                                             (int64_t)m.row_groups_cap * m.scratch_points / npts);
-      e = launch_logreg_fp32(m.x, m.y, m.n, m.p, m.hyper[0], Q, npts, ld, rg, m.part_g, m.part_ll, PE, G, pending, st,
-                             dependent);
+      e = launch_logreg_fp32(logreg_fp32_shape(m.n, npts, INT_MAX).variant, m.x, m.y, m.n, m.p, m.hyper[0], Q, npts, ld,
+                             rg, m.part_g, m.part_ll, PE, G, pending, st, dependent);
       if (e != cudaSuccess) return e;
       break;
     }
@@ -729,8 +734,8 @@ namespace gbn {
 cudaError_t launch_logreg_simt_scratch(const float* x, const float* y, int64_t n, int p, double prior_scale,
                                        const float* Q, int npts, int row_groups, float* part_g, double* part_ll,
                                        double* PE, float* G, cudaStream_t st) {
-  return launch_logreg_fp32(x, y, n, p, prior_scale, Q, npts, p, logreg_fp32_row_groups(n, p, npts, row_groups), part_g,
-                            part_ll, PE, G, nullptr, st, false);
+  return launch_logreg_fp32(logreg_fp32_shape(n, npts, row_groups).variant, x, y, n, p, prior_scale, Q, npts, p,
+                            logreg_fp32_row_groups(n, p, npts, row_groups), part_g, part_ll, PE, G, nullptr, st, false);
 }
 
 void horseshoe_finish_launch(const float* Q, int npts, int ld, int P, int64_t N, const float* part_gb, int splits,
