@@ -464,7 +464,8 @@ int gbn_create(gbn_handle* out, const gbn_model_desc* md, const gbn_config* cfg)
     gbn_destroy(h);
     return r == GBN_ERR_CUDA ? GBN_ERR_OOM : r;
   }
-  // launch shapes of the potential from the autotuner (GBN_AUTOTUNE=0 keeps the defaults)
+  // launch shapes of the potential: by rule, or from the autotuner (GBN_AUTOTUNE=0 keeps the defaults)
+  rule_shapes(m, C);
   {
     const char* at = getenv("GBN_AUTOTUNE");
     if (!(at && at[0] == '0')) {

@@ -8,10 +8,10 @@ namespace gbn {
 
 struct AdvParams;
 
-// Launch shapes of the potential kernels, chosen by autotune_potential (defaults before tuning) where they do not
-// change a result's bits, else by rule.  hier_cpb: chains (warps) per CTA of the hierarchical kernel; hs_tm: rows per thread of the horseshoe
-// residual GEMM (tile height 16 * hs_tm); hs_splits: row ranges of the horseshoe adjoint GEMM;
-// lr_rg: row groups of the FP32 logistic kernel (0: by rule, logreg_fp32_row_groups).
+// Launch shapes of the potential kernels: by rule (rule_shapes) where they change a result's bits, else chosen by
+// autotune_potential.  hier_cpb: chains (warps) per CTA of the hierarchical kernel; hs_tm: tile height 16 * hs_tm of the
+// horseshoe residual GEMM; hs_splits: row ranges of the horseshoe adjoint GEMM; lr_rg: row groups of the FP32 logistic
+// kernel (0: by rule, logreg_fp32_row_groups).
 struct TuneParams {
   int hier_cpb = 8;
   int hs_tm = 4;
@@ -132,10 +132,11 @@ void free_potential_scratch(ModelDev& m);
 // other potentials ignore it.  dependent: as launch_tick, for the potentials whose kernels take it
 cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, float* G,
                              const int32_t* pending, cudaStream_t st, bool fused_tick = false, bool dependent = false);
-// Times the candidate launch shapes of this model's potential at npts points (Q: any valid
-// [npts][D] positions; PE/G outputs) and stores the fastest in m.tune.  Decisions are cached per
-// process for each (device, family, shape, points), so every handle of a shape runs the same
-// arithmetic.  report receives "name=value ..." of the choice.
+// Sets the shapes that follow a rule on the model's sizes and the points of a handle.
+void rule_shapes(ModelDev& m, int points);
+// Applies GBN_TUNE, or times the candidate launch shapes of the hierarchical potential at npts points (Q: any
+// valid [npts][D] positions; PE/G outputs) and stores the fastest in m.tune, once per process for each
+// (device, family, shape, points).  report receives "name=value ..." of the shapes in use.
 cudaError_t autotune_potential(ModelDev& m, const float* Q, int npts, double* PE, float* G, cudaStream_t st,
                                std::string* report);
 // VJP: out[k] = cot[k] * grad U(z_k)

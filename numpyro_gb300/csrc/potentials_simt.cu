@@ -521,7 +521,10 @@ cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, 
         kernel<<<g1, threads, 0, st>>>(m.hs_xt, pad4(M), m.hs_bt, cp, M, npts, P, P, m.resid, cp, 0, m.y, m.part_rr, cp,
                                        pending);
       };
-      const bool large = npts >= 128 && m.n * P >= 1000000;  // as the tile height's rule (tune_params)
+      // as the tile height's rule (rule_shapes); three stages of 32 gain 4 us at the line (1000 x 1000 x 128: 59.5
+      // against 63.6) and as much below it where features are many (256 x 1000 x 128: 55.4 against 59.4), and lose 2
+      // where they are few (542 x 130 x 32: 28.7 against 26.7)
+      const bool large = npts >= 128 && m.n * P >= 1000000;
       if (tm == 2)
         large ? gemm1(hs_sgemm_nn_kernel<32, 32, 3>, 64) : gemm1(hs_sgemm_nn_kernel<32, 16, 4>, 64);
       else
@@ -588,6 +591,18 @@ std::string tune_report(const ModelDev& m) {
 }
 }  // namespace
 
+// The horseshoe's tile height and row ranges: by rule, not by timing, as both set the order of FP32 sums and a choice
+// made by a few launches' times made a model's results differ between processes.  Measured (us a potential, 300
+// shapes of 50 to 2,000 rows, 20 to 1,000 features, 1 to 256 points): 64 rows for large problems take 80.0 against 82.0
+// at 2000 x 1000 x 256 and 49.2 against 51.2 at 2000 x 500 x 256, at most 2 us either way below; the rule is 3.5 % from
+// the best of all on average, at most 2 us on small problems: 8 ranges are better than 4 from 129 rows on for few points (200 x 50: 22.6
+// against 24.6) and worse for 256 (25.6 against 24.6).
+void rule_shapes(ModelDev& m, int points) {
+  if (m.family != 3) return;
+  m.tune.hs_tm = points >= 128 && m.n * m.p >= 1000000 ? 4 : 2;
+  m.tune.hs_splits = m.n <= 64 ? 2 : (m.n <= 200 ? 4 : 8);
+}
+
 cudaError_t autotune_potential(ModelDev& m, const float* Q, int npts, double* PE, float* G, cudaStream_t st,
                                std::string* report) {
   int dev = 0;
@@ -596,7 +611,6 @@ cudaError_t autotune_potential(ModelDev& m, const float* Q, int npts, double* PE
   snprintf(key, sizeof(key), "%d|%d|%lld|%d|%d|%d|%d|%d|%g", dev, m.family, (long long)m.n, m.p, m.D, m.num_models,
            npts, m.precision, m.hyper[0]);
   std::lock_guard<std::mutex> lock(g_tune_mu);
-  auto it = g_tune_cache.find(key);
   cudaError_t e = ensure_potential_scratch(m, npts);
   if (e != cudaSuccess) return e;
   const char* forced = getenv("GBN_TUNE");  // "hier_cpb=16 hs_tm=2 hs_splits=8 lr_rg=32": fixed shapes
@@ -610,37 +624,26 @@ cudaError_t autotune_potential(ModelDev& m, const float* Q, int npts, double* PE
       m.tune.hs_splits = v;
     if ((p = strstr(forced, "lr_rg=")) && sscanf(p + 6, "%d", &v) == 1 && v >= 1 && v <= m.row_groups_cap)
       m.tune.lr_rg = v;
-  } else if (it != g_tune_cache.end()) {
-    m.tune = it->second;
-  } else {
-    std::vector<TuneParams> cand;
-    TuneParams t = m.tune;
-    if (m.family == 1) {
+  } else if (m.family == 1) {
+    auto it = g_tune_cache.find(key);
+    if (it != g_tune_cache.end()) {
+      m.tune = it->second;
+    } else {
+      float best = 1e30f;
+      TuneParams pick = m.tune;
       for (int cpb : {4, 8, 16}) {
-        t.hier_cpb = cpb;
-        cand.push_back(t);
+        m.tune.hier_cpb = cpb;
+        float ms = 0.0f;
+        e = time_potential(m, Q, npts, PE, G, st, 3, &ms);
+        if (e != cudaSuccess) return e;
+        if (ms < best) {
+          best = ms;
+          pick = m.tune;
+        }
       }
-    } else if (m.family == 3) {
-      // By rule, not by timing: both shapes set the order of FP32 sums, and a choice made by a few
-      // launches' times made a model's results differ between processes.
-      t.hs_tm = npts >= 128 && (int64_t)m.n * m.p >= 1000000 ? 4 : 2;
-      t.hs_splits = m.n <= 64 ? 2 : (m.n <= 200 ? 4 : 8);
-      cand.push_back(t);
+      m.tune = pick;
+      g_tune_cache[key] = pick;
     }
-    float best = 1e30f;
-    TuneParams pick = m.tune;
-    for (const TuneParams& c : cand) {
-      m.tune = c;
-      float ms = 0.0f;
-      e = time_potential(m, Q, npts, PE, G, st, 3, &ms);
-      if (e != cudaSuccess) return e;
-      if (ms < best) {
-        best = ms;
-        pick = c;
-      }
-    }
-    m.tune = pick;
-    g_tune_cache[key] = pick;
   }
   if (report) *report = tune_report(m);
   return cudaSuccess;

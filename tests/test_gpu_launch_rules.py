@@ -5,7 +5,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from numpyro_gb300 import NUTS, models  # noqa: E402
+from numpyro_gb300 import NUTS, datasets, models  # noqa: E402
 
 
 def _both(model, z, monkeypatch):
@@ -27,6 +27,14 @@ def test_logreg_row_groups(n, p, C, monkeypatch):
     X = rng.standard_normal((n, p)).astype(np.float32)
     y = (rng.random(n) < 0.4).astype(np.float32)
     _both(models.LogisticRegression(X, y), (0.1 * rng.standard_normal((C, p))).astype(np.float32), monkeypatch)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,p,C", [(64, 20, 3), (65, 50, 3), (200, 30, 128), (201, 96, 2), (1000, 1000, 127), (1000, 1000, 128)])
+def test_horseshoe_tiles(n, p, C, monkeypatch):
+    X, y, _ = datasets.horseshoe_data(seed=n, n=n, p=p, nonzero=5)
+    z = (0.1 * np.random.default_rng(C).standard_normal((C, 2 * p + 2))).astype(np.float32)
+    _both(models.HorseshoeRegression(X, y), z, monkeypatch)
 
 
 def _logreg(n, p, seed):
