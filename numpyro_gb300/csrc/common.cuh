@@ -374,6 +374,7 @@ struct Group;
 
 template <>
 struct Group<32> {  // one warp per chain
+  static constexpr bool searches = true;  // step-size searches need its sums
   int tid;
   __device__ __forceinline__ void sync() const { __syncwarp(); }
   __device__ __forceinline__ FF sumff(FF v, double*) const {
@@ -410,6 +411,7 @@ struct Group<32> {  // one warp per chain
 
 template <>
 struct Group<256> {  // one CTA of 256 threads per chain; red must hold 16 doubles
+  static constexpr bool searches = true;
   int tid;
   __device__ __forceinline__ void sync() const { __syncthreads(); }
   // warp butterflies, then every thread folds the 8 warp pairs in the same order

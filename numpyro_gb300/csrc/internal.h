@@ -102,7 +102,8 @@ void launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool 
                     bool dependent);
 cudaError_t launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order,
                                    int C, int D, int maxd, bool nuts, bool dense, cudaStream_t st);
-// searches: a warmup window's end may start a step-size search in this run
+// searches: the handle's warmup searches for step sizes at window ends (after warmup too: the host does not know how
+// far the chains of a state have come)
 cudaError_t launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t* queue_head, int C, int D, bool nuts,
                                  bool searches, cudaStream_t st);
 void launch_init_uniform(const AdvParams* dP, int C, int D, int attempt, const int32_t* flag, cudaStream_t st);

@@ -687,12 +687,17 @@ struct Chain {
         if (g.tid == 0) P.s.mm_n[c] = 0;
       }
       if (P.adapt_step) {
-        if (P.heuristic) {
-          if (g.tid == 0) P.s.step_size[c] = step;
-          g.sync();
-          heur_begin(HC_WINDOW, (uint32_t)t);
-          started = true;
-        } else if (g.tid == 0) {
+        bool search = false;
+        if constexpr (Threads::searches) {
+          search = P.heuristic != 0;
+          if (search) {
+            if (g.tid == 0) P.s.step_size[c] = step;
+            g.sync();
+            heur_begin(HC_WINDOW, (uint32_t)t);
+            started = true;
+          }
+        }
+        if (!search && g.tid == 0) {
           ss[0] = 0.0; ss[1] = 0.0; ss[2] = 0.0; ss[3] = 0.0;
           ss[4] = log(10.0) + log((double)step);
         }

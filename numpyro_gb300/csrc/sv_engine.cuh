@@ -26,12 +26,12 @@
 
 namespace gbn {
 
-// The 256 element threads as a group: as Group<256>, on a named barrier.
+// The 256 element threads as a group: as Group<256>, on a named barrier, for the end of a transition.  It has no sums,
+// which only step-size searches need there: runs of a handle that has them take persistent_sv_kernel.
 struct SvGroup {
+  static constexpr bool searches = false;
   int tid;
   __device__ __forceinline__ void sync() const { asm volatile("bar.sync 2, 256;" ::: "memory"); }
-  __device__ __forceinline__ FF sumff(FF v, double*) const { return v; }    // not used outside the leaf loop
-  __device__ __forceinline__ void sum2ff(FF&, FF&, double*) const {}
 };
 
 struct SvEngineSmem {
