@@ -212,7 +212,7 @@ __device__ __forceinline__ void hier_run_chain(const AdvParams& P, const HierVie
       int leaf = 0;
       bool sub_div = false, sub_turning = false;
       do {
-        if (depth > 4 && (leaf == 1 || (leaf & 31) == 0))  // lane l: leaf l of this block of 32
+        if (depth > 4 && (leaf == 1 || ((leaf & 31) == 0 && leaf > 0)))  // lane l: leaf l of this block of 32
           wl = hier_draw(P.seed, cid, n, P_LEAF, depth, (leaf & ~31) + lane).x;
         // ------------------------------------------------------ leapfrog to the new position
 #pragma unroll
