@@ -2,7 +2,7 @@
 //
 //   l = X b;  U = sum_n [softplus(l_n) - y_n l_n] + prior;  dU/db = X^T (sigmoid(l) - y) + prior
 // Fused per row tile: logits -> (softplus, sigmoid) -> gradient, so no logit reaches memory.  A CTA
-// owns CT chains and a strided set of RT-row tiles; a thread holds 4 RG rows x 4 CG chains of logits.
+// owns CT chains and a strided set of 64-row tiles; a thread holds 4 rows x 4 CG chains of logits.
 //
 // Bound: FP32 instruction issue.  A logit costs 2 p fused multiply-adds and ~60 instructions of expf, log1pf
 // and reciprocal (~100 with the compiler's division: 1 + e^-|l| lies in [1, 2], so the reciprocal needs no
@@ -57,33 +57,32 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) 
                : "memory");
 }
 
-// CT chains, NTH threads, RG groups of 4 rows and CG groups of 4 chains a thread in the logit phase,
-// 4 CG chains x 4 FG features a thread in the gradient phase, SP floats a row of the X tile (32 or 64),
-// NB tile buffers.
-template <int CT, int NTH, int RG, int CG, int FG, int SP, int NB>
+// CT chains, NTH threads, 4 rows x 4 CG chains a thread in the logit phase, 4 CG chains x 4 features a thread in the
+// gradient phase, SP floats a row of the X tile (32 or 64), two tile buffers.
+template <int CT, int NTH, int CG, int SP>
 struct LogregTile {
-  static constexpr int TX = CT / (4 * CG), TY = NTH / TX, RT = 4 * RG * TY;
+  static constexpr int TX = CT / (4 * CG), TY = NTH / TX, RT = 4 * TY;
   static constexpr size_t bytes(int dp) {
-    return sizeof(float) * (size_t)(NB * RT * SP + dp * CT + RT * CT + NB * RT) + sizeof(double) * (NTH / 32) * CT;
+    return sizeof(float) * (size_t)(2 * RT * SP + dp * CT + RT * CT + 2 * RT) + sizeof(double) * (NTH / 32) * CT;
   }
 };
 
-template <int CT, int NTH, int RG, int CG, int FG, int SP, int NB, int MINB>
+template <int CT, int NTH, int CG, int SP, int MINB>
 __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs A) {
-  using T = LogregTile<CT, NTH, RG, CG, FG, SP, NB>;
-  constexpr int TX = T::TX, TY = T::TY, RT = T::RT;
+  using T = LogregTile<CT, NTH, CG, SP>;
+  constexpr int TX = T::TX, RT = T::RT;
   extern __shared__ __align__(16) float lr_smem[];
   const int p = A.p, nc = (p + 3) >> 2;
-  float* const xs = lr_smem;                 // [NB][RT][SP], chunk c of row r at c ^ ((r >> 2) & 7)
-  float* const es = xs + NB * RT * SP;       // [RT][CT]
-  float* const ys = es + RT * CT;            // [NB][RT]
-  double* const lls = reinterpret_cast<double*>(ys + NB * RT);  // [NTH / 32][CT]
+  float* const xs = lr_smem;                 // [2][RT][SP], chunk c of row r at c ^ ((r >> 2) & 7)
+  float* const es = xs + 2 * RT * SP;        // [RT][CT]
+  float* const ys = es + RT * CT;            // [2][RT]
+  double* const lls = reinterpret_cast<double*>(ys + 2 * RT);  // [NTH / 32][CT]
   float* const bs = reinterpret_cast<float*>(lls + (NTH / 32) * CT);  // [4 nc][CT]
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int c0 = blockIdx.x * CT, rg = blockIdx.y, groups = gridDim.y;
   const int64_t ntiles = (A.n + RT - 1) / RT;
 
-  for (int k = tid; k < NB * RT * SP; k += NTH) xs[k] = 0.0f;  // features past p stay zero
+  for (int k = tid; k < 2 * RT * SP; k += NTH) xs[k] = 0.0f;  // features past p stay zero
   __syncthreads();
   auto load_tile = [&](int64_t tile, int buf) {
     float* const dst = xs + buf * RT * SP;
@@ -115,16 +114,16 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  // Gradient phase: a thread owns 4 CG chains x 4 FG features and takes the rows in order, so the sum of
+  // Gradient phase: a thread owns 4 CG chains x 4 features and takes the rows in order, so the sum of
   // an output does not depend on the tile's shape (only on which 64-row tiles a row group holds).
-  const int dgn = (nc + FG - 1) / FG, outs = TX * dgn;
+  const int outs = TX * nc;
   const int gc = tid % TX, gd = tid / TX;
-  static_assert(TX * (SP / (4 * FG)) <= NTH, "an output tile per thread");
-  float2 gacc[2 * CG][4 * FG];  // pairs of chains
+  static_assert(TX * (SP / 4) <= NTH, "an output tile per thread");
+  float2 gacc[2 * CG][4];  // pairs of chains
 #pragma unroll
   for (int i = 0; i < 2 * CG; ++i)
 #pragma unroll
-    for (int j = 0; j < 4 * FG; ++j) gacc[i][j] = make_float2(0.0f, 0.0f);
+    for (int j = 0; j < 4; ++j) gacc[i][j] = make_float2(0.0f, 0.0f);
   double ll[4 * CG];
 #pragma unroll
   for (int j = 0; j < 4 * CG; ++j) ll[j] = 0.0;
@@ -141,25 +140,22 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
     const int c = k / (4 * nc), d = k % (4 * nc);
     bs[d * CT + c] = (d < p && c0 + c < A.npts) ? A.q[(size_t)(c0 + c) * A.ld + d] : 0.0f;
   }
-  for (int64_t tile = rg; tile < ntiles; tile += groups, buf ^= NB - 1) {
+  for (int64_t tile = rg; tile < ntiles; tile += groups, buf ^= 1) {
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();  // this tile has landed; every thread is done with the other buffer and with E
-    if (NB == 2 && tile + groups < ntiles) load_tile(tile + groups, buf ^ 1);
+    if (tile + groups < ntiles) load_tile(tile + groups, buf ^ 1);
     const float* const xb = xs + buf * RT * SP;
     // ------------------------------------------------ logits
-    float2 acc[4 * RG][2 * CG];  // pairs of chains
+    float2 acc[4][2 * CG];  // pairs of chains
 #pragma unroll
-    for (int i = 0; i < 4 * RG; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 2 * CG; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
     for (int c = 0; c < nc; ++c) {
-      float4 xv[4 * RG];
+      float4 xv[4];
 #pragma unroll
-      for (int g = 0; g < RG; ++g)
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          xv[4 * g + i] = *reinterpret_cast<const float4*>(xb + (4 * (g * TY + ty) + i) * SP +
-                                                           ((c ^ ((g * TY + ty) & 7)) << 2));
+      for (int i = 0; i < 4; ++i)
+        xv[i] = *reinterpret_cast<const float4*>(xb + (4 * ty + i) * SP + ((c ^ (ty & 7)) << 2));
 #pragma unroll
       for (int dd = 0; dd < 4; ++dd) {
         float2 b[2 * CG];
@@ -170,7 +166,7 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
           b[2 * h + 1] = make_float2(b4.z, b4.w);
         }
 #pragma unroll
-        for (int i = 0; i < 4 * RG; ++i) {
+        for (int i = 0; i < 4; ++i) {
           const float xa = dd == 0 ? xv[i].x : (dd == 1 ? xv[i].y : (dd == 2 ? xv[i].z : xv[i].w));
 #pragma unroll
           for (int j = 0; j < 2 * CG; ++j) acc[i][j] = __ffma2_rn(make_float2(xa, xa), b[j], acc[i][j]);
@@ -179,63 +175,53 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
     }
     // ------------------------------------------------ softplus and sigmoid
     const int64_t left = A.n - tile * RT;
+    float llt[4 * CG];
 #pragma unroll
-    for (int g = 0; g < RG; ++g) {
-      float llt[4 * CG];
+    for (int j = 0; j < 4 * CG; ++j) llt[j] = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 4 * CG; ++j) llt[j] = 0.0f;
+    for (int i = 0; i < 4; ++i) {
+      const int r = 4 * ty + i;
+      const float yy = ys[buf * RT + r];
+      const bool in = r < left;
+      float ev[4 * CG];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = 4 * (g * TY + ty) + i;
-        const float yy = ys[buf * RT + r];
-        const bool in = r < left;
-        float ev[4 * CG];
-#pragma unroll
-        for (int j = 0; j < 4 * CG; ++j) {
-          const float l = (j & 1) ? acc[4 * g + i][j >> 1].y : acc[4 * g + i][j >> 1].x;
-          const float t = expf(-fabsf(l));
-          const float sp = fmaxf(l, 0.0f) + log1pf(t);
-          const float inv = recip_1_2(1.0f + t);
-          const float sig = (l >= 0.0f) ? inv : t * inv;
-          ev[j] = in ? sig - yy : 0.0f;
-          llt[j] += in ? sp - yy * l : 0.0f;
-        }
-#pragma unroll
-        for (int h = 0; h < CG; ++h)
-          *reinterpret_cast<float4*>(es + r * CT + h * (CT / CG) + 4 * tx) =
-              make_float4(ev[4 * h], ev[4 * h + 1], ev[4 * h + 2], ev[4 * h + 3]);
+      for (int j = 0; j < 4 * CG; ++j) {
+        const float l = (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x;
+        const float t = expf(-fabsf(l));
+        const float sp = fmaxf(l, 0.0f) + log1pf(t);
+        const float inv = recip_1_2(1.0f + t);
+        const float sig = (l >= 0.0f) ? inv : t * inv;
+        ev[j] = in ? sig - yy : 0.0f;
+        llt[j] += in ? sp - yy * l : 0.0f;
       }
 #pragma unroll
-      for (int j = 0; j < 4 * CG; ++j) ll[j] = CT <= 16 && tile == rg ? f2d(llt[j]) : ll[j] + f2d(llt[j]);  // few-chain tiles: no addition of 0
+      for (int h = 0; h < CG; ++h)
+        *reinterpret_cast<float4*>(es + r * CT + h * (CT / CG) + 4 * tx) =
+            make_float4(ev[4 * h], ev[4 * h + 1], ev[4 * h + 2], ev[4 * h + 3]);
     }
+#pragma unroll
+    for (int j = 0; j < 4 * CG; ++j)  // few-chain tiles: the first sum is not added to 0
+      ll[j] = CT <= 16 && tile == rg ? f2d(llt[j]) : ll[j] + f2d(llt[j]);
     __syncthreads();
     // ------------------------------------------------ gradient
     if (tid < outs) {
 #pragma unroll 2
       for (int r = 0; r < RT; ++r) {
         float2 e[2 * CG];
-        float xf[4 * FG];
+        float xf[4];
 #pragma unroll
         for (int h = 0; h < CG; ++h) {
           const float4 e4 = *reinterpret_cast<const float4*>(es + r * CT + h * (CT / CG) + 4 * gc);
           e[2 * h] = make_float2(e4.x, e4.y);
           e[2 * h + 1] = make_float2(e4.z, e4.w);
         }
+        const float4 x4 = *reinterpret_cast<const float4*>(xb + r * SP + ((gd ^ ((r >> 2) & 7)) << 2));
+        xf[0] = x4.x; xf[1] = x4.y; xf[2] = x4.z; xf[3] = x4.w;
 #pragma unroll
-        for (int f = 0; f < FG; ++f) {
-          const float4 x4 =
-              *reinterpret_cast<const float4*>(xb + r * SP + (((gd * FG + f) ^ ((r >> 2) & 7)) << 2));
-          xf[4 * f] = x4.x; xf[4 * f + 1] = x4.y; xf[4 * f + 2] = x4.z; xf[4 * f + 3] = x4.w;
-        }
-#pragma unroll
-        for (int j = 0; j < 4 * FG; ++j)
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
           for (int i = 0; i < 2 * CG; ++i) gacc[i][j] = __ffma2_rn(e[i], make_float2(xf[j], xf[j]), gacc[i][j]);
       }
-    }
-    if (NB == 1 && tile + groups < ntiles) {
-      __syncthreads();
-      load_tile(tile + groups, 0);
     }
   }
   // ------------------------------------------------ the CTA's partials
@@ -244,12 +230,9 @@ __global__ void __launch_bounds__(NTH, MINB) logreg_fp32_kernel(const LogregArgs
     for (int i = 0; i < 4 * CG; ++i) {
       const int c = c0 + (i >> 2) * (CT / CG) + 4 * gc + (i & 3);
       if (c >= A.npts) continue;
-#pragma unroll
-      for (int f = 0; f < FG; ++f) {
-        const float2* const v = gacc[i >> 1] + 4 * f;
-        *reinterpret_cast<float4*>(A.part_g + ((size_t)rg * A.npts + c) * 64 + 4 * (gd * FG + f)) =
-            (i & 1) ? make_float4(v[0].y, v[1].y, v[2].y, v[3].y) : make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
-      }
+      const float2* const v = gacc[i >> 1];
+      *reinterpret_cast<float4*>(A.part_g + ((size_t)rg * A.npts + c) * 64 + 4 * gd) =
+          (i & 1) ? make_float4(v[0].y, v[1].y, v[2].y, v[3].y) : make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
     }
   }
   // Across the lanes of a warp that share chains.  An SM starts an FP64 instruction every 19 cycles, so the lanes first
@@ -409,39 +392,38 @@ inline int logreg_fp32_row_groups(int64_t n, int p, int npts, int want) {
   return (int)pick;
 }
 
-template <int CT, int NTH, int RG, int CG, int FG, int NB32, int NB64, int MINB>
+template <int CT, int NTH, int CG, int MINB>
 static cudaError_t logreg_fp32_launch_variant(const LogregArgs& A, int row_groups, bool attr, cudaStream_t st,
                                               bool dependent) {
   const int dp = (A.p + 3) / 4 * 4;
   const dim3 grid((A.npts + CT - 1) / CT, row_groups);
   if (attr) {  // the shared-memory limit, at the most features each instance takes
-    cudaError_t e = cudaFuncSetAttribute(logreg_fp32_kernel<CT, NTH, RG, CG, FG, 32, NB32, MINB>,
+    cudaError_t e = cudaFuncSetAttribute(logreg_fp32_kernel<CT, NTH, CG, 32, MINB>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)LogregTile<CT, NTH, RG, CG, FG, 32, NB32>::bytes(32));
+                                         (int)LogregTile<CT, NTH, CG, 32>::bytes(32));
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(logreg_fp32_kernel<CT, NTH, RG, CG, FG, 64, NB64, MINB>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)LogregTile<CT, NTH, RG, CG, FG, 64, NB64>::bytes(64));
+      e = cudaFuncSetAttribute(logreg_fp32_kernel<CT, NTH, CG, 64, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)LogregTile<CT, NTH, CG, 64>::bytes(64));
     return e;
   }
   if (dp <= 32)
-    return launch_tick(logreg_fp32_kernel<CT, NTH, RG, CG, FG, 32, NB32, MINB>, grid, NTH,
-                       LogregTile<CT, NTH, RG, CG, FG, 32, NB32>::bytes(dp), st, dependent, A);
-  return launch_tick(logreg_fp32_kernel<CT, NTH, RG, CG, FG, 64, NB64, MINB>, grid, NTH,
-                     LogregTile<CT, NTH, RG, CG, FG, 64, NB64>::bytes(dp), st, dependent, A);
+    return launch_tick(logreg_fp32_kernel<CT, NTH, CG, 32, MINB>, grid, NTH, LogregTile<CT, NTH, CG, 32>::bytes(dp), st,
+                       dependent, A);
+  return launch_tick(logreg_fp32_kernel<CT, NTH, CG, 64, MINB>, grid, NTH, LogregTile<CT, NTH, CG, 64>::bytes(dp), st,
+                     dependent, A);
 }
 
 // variant < 0: sets every variant's shared-memory limit on the current device
 static cudaError_t logreg_fp32_launch(int variant, const LogregArgs& A, int row_groups, cudaStream_t st, bool dependent) {
   const bool attr = variant < 0;
   cudaError_t e = cudaSuccess;
-  if (attr || variant == 0) e = logreg_fp32_launch_variant<8, 32, 1, 1, 1, 2, 2, 6>(A, row_groups, attr, st, dependent);
+  if (attr || variant == 0) e = logreg_fp32_launch_variant<8, 32, 1, 6>(A, row_groups, attr, st, dependent);
   if ((attr && e == cudaSuccess) || variant == 1)
-    e = logreg_fp32_launch_variant<16, 64, 1, 1, 1, 2, 2, 5>(A, row_groups, attr, st, dependent);
+    e = logreg_fp32_launch_variant<16, 64, 1, 5>(A, row_groups, attr, st, dependent);
   if ((attr && e == cudaSuccess) || variant == 2)
-    e = logreg_fp32_launch_variant<64, 256, 1, 1, 1, 2, 2, 2>(A, row_groups, attr, st, dependent);
+    e = logreg_fp32_launch_variant<64, 256, 1, 2>(A, row_groups, attr, st, dependent);
   if ((attr && e == cudaSuccess) || variant == 3)
-    e = logreg_fp32_launch_variant<128, 256, 1, 2, 1, 2, 2, 2>(A, row_groups, attr, st, dependent);
+    e = logreg_fp32_launch_variant<128, 256, 2, 2>(A, row_groups, attr, st, dependent);
   return e;
 }
 
