@@ -631,7 +631,7 @@ def main():
     # DRAM bytes (read + write) of one launch of the dominant kernel, from the ncu capture summarised
     # in profiles/ for this kernel at 1024 chains
     traffic, traffic_src = profiled_traffic(
-        "logreg_tc_kernel_covtype_1024chains" if precision == "bf16x3" else "logreg_simt_kernel_covtype_1024chains",
+        "logreg_tc_kernel_covtype_1024chains" if precision == "bf16x3" else "logreg_fp32_kernel_covtype_1024chains",
         X.shape[0])
     if C != 1024:
         traffic, traffic_src = None, None

@@ -7,8 +7,8 @@
 // Chain<32> (nuts_engine.cu) and hier_nc_potential_warp, term for term and in the same order, so
 // its draws are bit-identical to the tick engine's.
 //
-// What bounds it: the dependent instructions of one leaf for a few chains (3,500 cycles), the FP64
-// pipe and instruction fetch for thousands.  The sums of a leaf (potential 3, kinetic energy 1, U-turn
+// What bounds it: the dependent instructions of one leaf for a few chains (4,300 cycles with its share of the
+// transition's end), the FP64 pipe and instruction fetch for thousands.  The sums of a leaf (potential 3, kinetic energy 1, U-turn
 // 2 per check) are float-float: a butterfly costs 5 x (2 shuffles + 11 FP32 adds).  Summed together,
 // the values are dealt to lane groups in the first two steps (warp_sum3ff), so three of them cost 6
 // additions instead of 15, in two rounds per leaf (the potential's sums, then the energy with the
@@ -27,7 +27,7 @@ __device__ __forceinline__ FF ff_from_lane(FF v, int src) {
   return FF{__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src)};
 }
 
-// Out of line: one copy of the generator per kernel instead of K + 3.  With 16 warps of an SM at
+// Out of line: one copy of the generator per kernel instead of K + 3.  With 12 warps of an SM at
 // different places of the tree, the size of the leaf loop's code is what the instruction cache sees.
 __device__ __noinline__ uint4 hier_draw(Seed s, uint32_t chain, uint32_t n, uint32_t purpose, int idx, int sub) {
   return draw(s, chain, n, purpose, (uint32_t)idx, (uint32_t)sub);

@@ -11,7 +11,7 @@
 // shared memory as 16-byte words; X tiles arrive by cp.async one tile ahead, rows swizzled by groups of
 // four so that the eight lanes of a load phase meet eight bank groups.
 // Measured at 581,012 x 55 x 1,024 chains: 5.52 ms (64 x 64 tile, 4 x 4 a thread, X through registers and a
-// transposed copy) -> 3.64 ms = 36 TFLOP/s.  8 x 8 logits a thread with 8 warps per SM: 3.85; scalar
+// transposed copy) -> 3.65 ms = 36 TFLOP/s.  8 x 8 logits a thread with 8 warps per SM: 3.85; scalar
 // multiply-adds: 3.86.
 // Sums: a chain's log-likelihood of four consecutive rows in FP32, then FP64 over the thread's rows, across threads
 // and across CTAs.  (Compensated FP32 pairs within a CTA leave the potential 2^-48 off instead of 2^-53 and are
@@ -27,7 +27,7 @@ namespace gbn {
 
 // 1 / d for d in [1, 2], rounded to nearest: one Newton-Raphson step on the approximate reciprocal with
 // the residual exact in a fused multiply-add (Markstein, IBM J. Res. Dev. 34, 1990).  Equal to 1.0f / d
-// for each of the 2^23 + 1 floats of the range (compared on the GPU).
+// for each of the 2^23 + 1 floats of the range (tests/test_gpu_reciprocal.py compares them all).
 __device__ __forceinline__ float recip_1_2(float d) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
