@@ -552,8 +552,9 @@ static cudaError_t upload_params(gbn_handle h, cudaStream_t st) {
 // issues the same launches with the same arguments; the kernels read their parameters from
 // device memory).
 constexpr int TICK_BATCH = 16;
-// dependent: each kernel may start while the one before it ends (launch_tick).
+// dependent: each kernel may start while the one before it ends (launch_tick), where that pays.
 static cudaError_t launch_tick_batch(gbn_handle h, cudaStream_t st, bool dependent) {
+  dependent = dependent && tick_dependent(h->m, h->C);
   for (int k = 0; k < TICK_BATCH; ++k) {
     const int parity = k & 1;
     launch_advance(h->dP, h->C, h->D, h->cta_per_chain, h->hp.dense != 0, parity, st, dependent);

@@ -133,6 +133,8 @@ void free_potential_scratch(ModelDev& m);
 // other potentials ignore it.  dependent: as launch_tick, for the potentials whose kernels take it
 cudaError_t launch_potential(ModelDev& m, const float* Q, int npts, double* PE, float* G,
                              const int32_t* pending, cudaStream_t st, bool fused_tick = false, bool dependent = false);
+// Whether dependent launches shorten the tick loop of this model with that many chains.
+bool tick_dependent(const ModelDev& m, int points);
 // Sets the shapes that follow a rule on the model's sizes and the points of a handle.
 void rule_shapes(ModelDev& m, int points);
 // Applies GBN_TUNE, or times the candidate launch shapes of the hierarchical potential at npts points (Q: any

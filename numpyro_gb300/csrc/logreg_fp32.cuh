@@ -352,15 +352,19 @@ inline LogregShape logreg_fp32_shape(int64_t n, int npts, int max_groups) {
   return {0, 8};
 }
 // Row groups (CTAs of a chain group) by a rule on the sizes, as they set the order of FP32 sums: picked by timing, a
-// model's draws differed between processes.  One a tile for small data sets of up to LR_ORDERED_POINTS points, else the same number of tiles in
-// every group where that can be, and of the counts that put k = 1 to 8 CTAs on the busiest SM the largest (with
-// the shortest sums) within 1 % of the least cost:
-//   k (tiles of a CTA + 0.15) f + 0.004 for each group (the finish),
-// f what CTAs cost that do not fill an SM: one tile of 64 or 128 chains alone does not overlap its phases
-// (1.2; 64 chains of few features 1.5), 8 chains are a warp, so that fewer than 4 leave schedulers idle and more
-// overlap better (1 + 0.8 / k from 4 on).  16 chains, and 8 with many features, take 4 CTAs an SM.
-// Over 900 shapes of 8,193 to 581,012 rows, 5 to 55 features and 1 to 1,024 chains this is 0.5 % slower on average than
-// the best of up to 20 group counts (the best of three timed ones, as before: 1.8 %).  want > 0: at most that many.
+// model's draws differed between processes.  One a tile for small data sets of up to LR_ORDERED_POINTS points, else
+// the same number of tiles in every group where that can be, and of the counts that put one CTA on each SM or k = 1
+// to 8 on the busiest the largest (with the shortest sums) within 1 % of the least cost:
+//   64 and 128 chains   k (tiles of a CTA + 0.4) + 0.006 for each group (the finish).  In the tick loop the CTAs start beside
+//                       the state machine's, eight chains each, and go to the other SMs first: as many CTAs as
+//                       those have one each, f = 1.3 + 4 / p (1.5 at most) times as slow as two that overlap their
+//                       phases; more, up to one an SM, meet on one SM, k = 2 (45,000 rows x 50 features x 100 chains:
+//                       141 CTAs beside 13 take 5.8 ms for 60 ticks, 235 4.1; 60,000: 134 4.6, 235 5.1).
+//   8 chains            k (tiles + 0.15) (1 + 0.8 / k) + 0.004 a group, k = 4 at least: a CTA is a warp, fewer leave
+//                       schedulers idle and more overlap better.  16 chains, and 8 with many features: 4 CTAs an SM.
+// Against the best of up to 20 counts a potential alone is 1.1 % slower on average (900 shapes of 8,193 to 581,012
+// rows, 5 to 55 features, 1 to 1,024 chains; the best of three timed ones, as before: 1.8 %), a run 0.5 % (520
+// shapes of 8,256 to 90,000 rows, 20 to 1,024 chains).  want > 0: at most that many.
 inline int logreg_fp32_row_groups(int64_t n, int p, int npts, int want) {
   const int64_t tiles = (n + 63) / 64;
   if (tiles <= LR_ORDERED && want > 0) return (int)std::min<int64_t>(want, tiles);
@@ -372,25 +376,34 @@ inline int logreg_fp32_row_groups(int64_t n, int p, int npts, int want) {
     return (tiles + per - 1) / per;
   };
   if (want > 0) return (int)even(want);
-  const bool few_features = p <= 32;
-  if (s.variant == 1 || (s.variant == 0 && !few_features)) return (int)even(4 * LR_SMS / cgroups);
-  const double alone = s.variant == 2 && few_features ? 1.5 : 1.2;
-  const double group = s.variant == 2 && few_features ? 0.008 : 0.004;
+  if (s.variant == 1 || (s.variant == 0 && p > 32)) return (int)even(4 * LR_SMS / cgroups);
+  const bool few = s.variant == 0;
+  const int64_t beside = LR_SMS - std::min(LR_SMS, (npts + 7) / 8);  // SMs without a CTA of the state machine
+  const double alone = std::min(1.5, 1.3 + 4.0 / p);
   int64_t pick = 1;
   double least = 1e300;
-  for (int k = 1; k <= 8; ++k) {
-    const int64_t g = even((int64_t)k * LR_SMS / cgroups), per = (tiles + g - 1) / g;
-    double ctas = (double)((g * cgroups + LR_SMS - 1) / LR_SMS), f = ctas > 1.0 ? 1.0 : alone;
-    if (s.variant == 0) {
-      ctas = std::max(ctas, 4.0);
-      f = 1.0 + 0.8 / ctas;
+  for (int k = few ? 1 : 0; k <= 8; ++k) {
+    const int64_t room = k == 0 ? beside : (int64_t)k * LR_SMS;
+    if (k == 0 && room < cgroups) continue;
+    const int64_t g = even(room / cgroups), per = (tiles + g - 1) / g, ctas = g * cgroups;
+    const double busiest = (double)((ctas + LR_SMS - 1) / LR_SMS);
+    double cost;
+    if (few) {
+      const double b = std::max(busiest, 4.0);
+      cost = b * ((double)per + 0.15) * (1.0 + 0.8 / b) + 0.004 * (double)g;
+    } else {
+      cost = (ctas <= beside ? alone : std::max(busiest, 2.0)) * ((double)per + 0.4) + 0.006 * (double)g;
     }
-    const double cost = ctas * ((double)per + 0.15) * f + group * (double)g;
     if (cost < 1.01 * least) pick = g;
     least = std::min(least, cost);
   }
   return (int)pick;
 }
+// Whether the tick loop's kernels of such a model start while the one before them ends.  That takes 4 to 20 % off a run
+// of up to 512 chains.  With more the early CTAs crowd the SMs that the state machine's leave free: 1,000 rows x 1,024
+// chains take 1.36 ms for 60 ticks against 1.12, 5,000 x 2,000 3.43 against 3.25; from 2,000 rows up to 1,024 chains still gain
+// (1.50 against 1.60).
+inline bool logreg_fp32_dependent(int64_t n, int npts) { return npts <= 512 || (npts <= 1024 && n > 1024); }
 
 template <int CT, int NTH, int CG, int MINB>
 static cudaError_t logreg_fp32_launch_variant(const LogregArgs& A, int row_groups, bool attr, cudaStream_t st,

@@ -591,6 +591,10 @@ std::string tune_report(const ModelDev& m) {
 }
 }  // namespace
 
+bool tick_dependent(const ModelDev& m, int points) {
+  return m.family != 2 || m.tc || logreg_fp32_dependent(m.n, points);
+}
+
 // The horseshoe's tile height and row ranges: by rule, not by timing, as both set the order of FP32 sums and a choice
 // made by a few launches' times made a model's results differ between processes.  Measured (us a potential, 300
 // shapes of 50 to 2,000 rows, 20 to 1,000 features, 1 to 256 points): 64 rows for large problems take 80.0 against 82.0
