@@ -557,9 +557,11 @@ static cudaError_t launch_tick_batch(gbn_handle h, cudaStream_t st, bool depende
   dependent = dependent && tick_dependent(h->m, h->C);
   for (int k = 0; k < TICK_BATCH; ++k) {
     const int parity = k & 1;
-    launch_advance(h->dP, h->C, h->D, h->cta_per_chain, h->hp.dense != 0, parity, st, dependent);
-    cudaError_t e = launch_potential(h->m, h->e.Q, h->C, h->e.PE, h->e.G, h->counters + 2 * parity, st,
-                                     h->hp.lrf_part_g != nullptr || h->hp.hsf_part_gb != nullptr, dependent);
+    cudaError_t e =
+        launch_advance(h->dP, h->C, h->D, h->cta_per_chain, h->hp.dense != 0, parity, st, dependent);
+    if (e == cudaSuccess)
+      e = launch_potential(h->m, h->e.Q, h->C, h->e.PE, h->e.G, h->counters + 2 * parity, st,
+                           h->hp.lrf_part_g != nullptr || h->hp.hsf_part_gb != nullptr, dependent);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

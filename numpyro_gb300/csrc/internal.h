@@ -74,9 +74,10 @@ struct SvView {
 
 // Launches a kernel of the tick loop; dependent: it may start while its predecessor in the stream ends
 // (programmatic dependent launch, also when captured into a graph), for kernels that call tick_wait.
+// The result is the only report of a failure: a plain launch takes the last error.
 template <typename... P, typename... A>
-cudaError_t launch_tick(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool dependent,
-                        A... args) {
+[[nodiscard]] cudaError_t launch_tick(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                      bool dependent, A... args) {
   if (!dependent) {  // a plain launch costs the host a microsecond less
     kernel<<<grid, block, smem, st>>>(static_cast<P>(args)...);
     return cudaGetLastError();
@@ -98,8 +99,8 @@ inline int pad4(int v) { return (v + 3) & ~3; }
 
 // nuts_engine.cu
 // a CTA per chain when cta_per_chain or D > 1024, else a warp per chain
-void launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity, cudaStream_t st,
-                    bool dependent);
+[[nodiscard]] cudaError_t launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity,
+                                         cudaStream_t st, bool dependent);
 cudaError_t launch_persistent_hier(const AdvParams* dP, const HierView& hv, int32_t* queue_head, const int32_t* order,
                                    int C, int D, int maxd, bool nuts, bool dense, cudaStream_t st);
 // searches: the handle's warmup searches for step sizes at window ends (after warmup too: the host does not know how

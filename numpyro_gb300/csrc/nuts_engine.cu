@@ -1399,15 +1399,15 @@ cudaError_t launch_persistent_sv(const AdvParams* dP, const SvView& sv, int32_t*
   return cudaGetLastError();
 }
 
-void launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity, cudaStream_t st,
-                    bool dependent) {
+cudaError_t launch_advance(const AdvParams* dP, int C, int D, bool cta_per_chain, bool dense, int parity,
+                           cudaStream_t st, bool dependent) {
   if (!cta_per_chain && D <= 1024) {
     const int cpb = 8;
-    launch_tick(dense ? advance_kernel<32, true> : advance_kernel<32, false>, (C + cpb - 1) / cpb, 32 * cpb, 0, st,
-                dependent, dP, parity);
-  } else {  // dense mass needs a warp per chain
-    launch_tick(advance_kernel<256, false>, C, 256, 0, st, dependent, dP, parity);
+    return launch_tick(dense ? advance_kernel<32, true> : advance_kernel<32, false>, (C + cpb - 1) / cpb, 32 * cpb, 0,
+                       st, dependent, dP, parity);
   }
+  // dense mass needs a warp per chain
+  return launch_tick(advance_kernel<256, false>, C, 256, 0, st, dependent, dP, parity);
 }
 
 void launch_init_uniform(const AdvParams* dP, int C, int D, int attempt, const int32_t* flag, cudaStream_t st) {
